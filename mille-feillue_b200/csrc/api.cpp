@@ -375,7 +375,7 @@ int mf_spmv_bench(const mf_tiles *t, const double *x, double *y, int reps, doubl
 // --------------------------------------------------------------- solvers
 static int ensure_workspace(mf_tiles *t) {
     const size_t n16 = (size_t)t->tilem * 16;
-    const size_t need = 9 * n16 + 2 * 4 * (size_t)t->G + 64;  // 8 vectors + the FP32 pair
+    const size_t need = 9 * n16 + partial_words(t->G) + 64;  // 8 vectors + the FP32 pair, packets, norms
     if (t->ws.n < need) {
         if (t->ws.alloc(need)) return MF_ERR_NOMEM;
     }
@@ -416,7 +416,7 @@ static int true_residual_ws(mf_tiles *t, const double *b, const double *x, doubl
     WsView v = ws_view(t);
     int rc = launch_spmv(t, -1, x, v.q, 1, 0);
     if (rc) return rc;
-    double *out = v.partial + 2 * 4 * t->G;
+    double *out = v.partial + partial_words(t->G);
     if ((rc = launch_residual_norms(t->rowA, b, v.q, out, 0))) return rc;
     double h[2];
     MF_CUDA_TRY(cudaMemcpy(h, out, sizeof h, cudaMemcpyDeviceToHost));
@@ -439,7 +439,7 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     WsView v = ws_view(t);
     const size_t n16 = (size_t)t->tilem * 16;
     const int n = t->rowA;
-    MF_CUDA_TRY(cudaMemsetAsync(t->ws.p, 0, sizeof(double) * 9 * n16));
+    MF_CUDA_TRY(cudaMemsetAsync(t->ws.p, 0, sizeof(double) * (9 * n16 + partial_words(t->G))));
     MF_CUDA_TRY(cudaMemcpyAsync(v.b, b_dev, sizeof(double) * n, cudaMemcpyDeviceToDevice));
     MF_CUDA_TRY(cudaMemcpyAsync(v.x, x_dev, sizeof(double) * n, cudaMemcpyDeviceToDevice));
     MF_CUDA_TRY(cudaMemsetAsync(t->sync.p, 0, sizeof(uint32_t) * t->sync.n));

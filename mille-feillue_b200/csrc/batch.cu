@@ -60,7 +60,7 @@ struct mf_batch {
 namespace {
 
 constexpr int kBatchGroupDefault = 4;  // CTAs per system group (fastest of 4, 8, 16 on the 512-system set)
-// group sync words: arrive counter, error word, rank flags (32-byte aligned)
+// group sync words: error word, rank flags (32-byte aligned)
 size_t group_sync_words(int gs) { return (sync_words(gs) + 7) & ~(size_t)7; }
 
 // packed[poff_s + i] <-> ws vector of system s, row i (i < n_s)
@@ -160,7 +160,7 @@ int mf_batch_create(int count, const mf_csr *systems, const mf_options *opt_in, 
     if (B->ws.alloc((size_t)5 * B->ws_rows) || B->d_desc.alloc(count) || B->d_order.alloc(count) ||
         B->d_n.alloc(count) || B->d_voff.alloc(count) || B->d_poff.alloc(count) || B->d_queue.alloc(1) ||
         B->d_res.alloc(count) || B->d_sync.alloc((size_t)B->ngroups * group_sync_words(B->gs)) ||
-        B->d_partial.alloc((size_t)B->ngroups * 8 * B->gs)) {
+        B->d_partial.alloc((size_t)B->ngroups * partial_words(B->gs))) {
         delete B;
         return MF_ERR_NOMEM;
     }
@@ -229,6 +229,7 @@ int mf_batch_solve_cg_dev(mf_batch *B, const double *b, double *x, double tol, i
         MF_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         cudaMemsetAsync(B->d_queue.p, 0, sizeof(unsigned), s);
         cudaMemsetAsync(B->d_sync.p, 0, sizeof(uint32_t) * B->d_sync.n, s);
+        cudaMemsetAsync(B->d_partial.p, 0, sizeof(double) * B->d_partial.n, s);  // the packets' phase tags
         cudaMemsetAsync(B->ws.p, 0, sizeof(double) * 5 * B->ws_rows, s);
         k_scatter<<<std::min(B->count, 1024), 256, 0, s>>>(b, B->ws.p, B->d_voff.p, B->d_poff.p, B->d_n.p,
                                                           B->count, B->ws_rows, 0);

@@ -81,6 +81,34 @@ MF_DEV uint32_t ld_relaxed(const uint32_t *p) {
 MF_DEV void st_release(uint32_t *p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+MF_DEV void st_relaxed(uint32_t *p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+MF_DEV void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// A reduction packet: a value and its phase tag in one 16-byte access, which
+// is a single memory operation (.b128), so a reader that sees the tag has the
+// value. p is 16-byte aligned.
+MF_DEV void st_packet_relaxed(double *p, double v, uint64_t tag) {
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\t"
+        "mov.b128 t, {%1, %2};\n\t"
+        "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+        "l"(__double_as_longlong(v)), "l"(tag)
+        : "memory");
+}
+MF_DEV uint64_t ld_packet_relaxed(const double *p, double &v) {
+    long long lo;
+    uint64_t tag;
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\t"
+        "ld.relaxed.gpu.global.b128 t, [%2];\n\t"
+        "mov.b128 {%0, %1}, t;\n\t}"
+        : "=l"(lo), "=l"(tag)
+        : "l"(p)
+        : "memory");
+    v = __longlong_as_double(lo);
+    return tag;
+}
 MF_DEV void red_release_add(uint32_t *p, uint32_t v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }

@@ -12,7 +12,7 @@
 // Limits: n rounded up to a multiple of 16 must be <= MF_NOALLOC_MAX_ROWS
 // (131072) and the solver grid must have <= 1024 CTAs; larger systems return
 // MF_ERR_ARG with a message and are left to mf_solve_cg_dev. The scratch costs
-// about 5.1 MiB of device memory per device, taken when the module loads.
+// about 5.3 MiB of device memory per device, taken when the module loads.
 //
 // Set-up: the first call on each device (with that device current) looks up
 // the scratch address with cudaGetSymbolAddress. Make that first call before
@@ -36,7 +36,7 @@ namespace {
 
 constexpr int NA_MAX_G = 1024;
 constexpr size_t NA_VEC_WORDS = 5 * (size_t)MF_NOALLOC_MAX_ROWS;  // b, x, r, d, q
-constexpr size_t NA_PART_WORDS = 2 * 4 * (size_t)NA_MAX_G + 64;   // reduction slots + norms
+constexpr size_t NA_PART_WORDS = 2 * PACKET_STRIDE * (size_t)NA_MAX_G + 64;  // reduction packets (partial_words) + norms
 constexpr size_t NA_SYNC_U32 =
     (size_t)SYNC_FLAGS + (size_t)NA_MAX_G * FLAG_STRIDE + 32 + sizeof(DevResult) / 4 + 8;
 constexpr size_t NA_WORDS = NA_VEC_WORDS + NA_PART_WORDS + (NA_SYNC_U32 + 1) / 2;
@@ -104,9 +104,10 @@ extern "C" int mf_solve_cg_dev_noalloc(mf_tiles *t, const double *b_dev, double 
     DevResult *dres = reinterpret_cast<DevResult *>(sync + sync_words(t->G));
 
     // Must start at zero: the vectors (their padding rows past n are read by
-    // the SpMV and the dot products), the grid-sync counters, the CTA epoch
-    // flags, the error word and the result record.
+    // the SpMV and the dot products), the reduction packets' tags, the CTA
+    // epoch flags, the error word and the result record.
     MF_CUDA_TRY(cudaMemsetAsync(w, 0, sizeof(double) * 5 * n16));
+    MF_CUDA_TRY(cudaMemsetAsync(partial, 0, sizeof(double) * partial_words(t->G)));
     MF_CUDA_TRY(cudaMemsetAsync(sync, 0, sizeof(uint32_t) * (sync_words(t->G) + sizeof(DevResult) / 4 + 8)));
     MF_CUDA_TRY(cudaMemcpyAsync(vb, b_dev, sizeof(double) * n, cudaMemcpyDeviceToDevice));
     MF_CUDA_TRY(cudaMemcpyAsync(vx, x_dev, sizeof(double) * n, cudaMemcpyDeviceToDevice));
@@ -150,7 +151,7 @@ extern "C" int mf_solve_cg_dev_noalloc(mf_tiles *t, const double *b_dev, double 
     R.rel_residual_true = NAN;
     if (!err[0] && opt.check_true_residual) {
         // A x into the q slot, the two norms into the tail of the partials
-        double *out = partial + 2 * 4 * (size_t)t->G;
+        double *out = partial + partial_words(t->G);
         if ((rc = launch_spmv(t, -1, vx, vq, 1, 0))) return rc;
         if ((rc = launch_residual_norms(n, vb, vq, out, 0))) return rc;
         double h[2];

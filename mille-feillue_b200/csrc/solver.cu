@@ -10,11 +10,11 @@
 // then y += sum; FP64 tiles use non-fused multiply/add, so the result is
 // bit-identical to that loop.
 //
-// Grid-wide dot products: each CTA reduces its partial in a fixed order,
-// stores it in a double-buffered slot, then arrives on a monotonic counter
-// with a release add; every CTA waits with acquire loads until all G CTAs
-// arrived, then sums the G partials in the same fixed order, so all CTAs
-// hold the identical value (no grid.sync, no kernel boundary). Vector halos
+// Grid-wide dot products: each CTA reduces its partial in a fixed order and
+// stores it with a phase tag as one 16-byte packet in a double-buffered slot;
+// every CTA polls the G packets until all carry the tag and sums them in the
+// same fixed order, so all CTAs hold the identical value (no grid.sync, no
+// kernel boundary). Vector halos
 // between iterations use per-CTA epoch flags (st.release / ld.acquire) that
 // only the CTAs whose rows a CTA reads are waited on. Every wait is bounded
 // by %globaltimer; on expiry the kernel records MF_ERR_TIMEOUT and returns.
@@ -47,7 +47,7 @@ struct __align__(16) Smem {
     uint8_t res_tag[STAGES];  // 1 + layout whose slab (index = stage) the stage holds; 0: none
     int slab0[KMAX_LAYOUTS], slab1[KMAX_LAYOUTS];
     double red[NWARPS + 1][4];
-    double bres[4];
+    double chunk[PACKET_VALUES * MAX_CHUNKS];  // group_sum: sums of 32 CTAs' packets
     uint8_t head[KMAX_LAYOUTS][STAGES][ISSUE_REC];
 };
 
@@ -669,47 +669,64 @@ __device__ bool cta_spmv(const KParams &P, int lay, const void *xv, Smem &S, uin
     return cta_spmv_src<MIXED, Epi, GB>(L, C, xv, S, dyn, pp, epi);
 }
 
-// Block reduction of NV partials in a fixed order, then the grid-wide sum.
 // A group of G CTAs that synchronize with each other (the whole grid for the
 // single-system kernels, a slice of it for the batched one).
 struct Ctx {
     uint32_t *sync;
-    double *partial;
+    double *partial;  // reduction packets, zero at launch
     int G, rank;
     uint64_t limit_ns;
 };
 
+// Sums NV partials over the block and then over the group, in fixed orders:
+// every CTA holds the identical sums. Thread k < NV adds the warps' shares of
+// value k and stores {share of this CTA, phase tag} as one 16-byte packet
+// (slot [phase & 1][rank][k]). Then each warp takes chunks of 32 CTAs of one
+// value, polls one packet a lane until it carries the tag, and adds the
+// chunk by a shuffle tree; the chunks are added in ascending order.
+// Latency-bound: a packet costs one store and one load through L2, where an
+// arrival counter costs a release, the wait on the counter and a second trip
+// for the partials (148 CTAs, 512 threads, one value: 1.4 us against 2.3).
+// Packets of different CTAs lie a 128-byte line apart: with 16 bytes between
+// them the polls collide (2.4 us).
+// Two slots are enough: a CTA writes phase p + 2 only after it saw every
+// CTA's packet of phase p + 1, which each sends after it read the packets of
+// phase p. The sum orders no memory but its own packets: vectors that one CTA
+// writes and another reads go through publish and wait_deps. It does keep a
+// CTA from overwriting what another is still reading: reads whose values went
+// into a CTA's packet (or landed in its ring) are complete when the packet is
+// stored.
 template <int NV>
 __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (&out)[NV], uint32_t &phase) {
+    static_assert(NV <= PACKET_VALUES, "one packet per value");
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    double t[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        t[k] = v[k];
+        double t = v[k];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) S.red[w][k] = t;
     }
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) S.red[w][k] = t[k];
     __syncthreads();
-    const int G = X.G;
-    const int slot = phase & 1;
-    if (tid == 0) {
-        double p[NV];
+    const uint64_t tag = (uint64_t)phase + 1u;
+    double *slot = X.partial + (size_t)(phase & 1u) * X.G * PACKET_STRIDE;
+    if (tid < NV) {
+        double p = 0.0;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            p[k] = 0.0;
-            for (int q = 0; q <= NWARPS; ++q) p[k] += S.red[q][k];
-            X.partial[((size_t)slot * G + X.rank) * 4 + k] = p[k];
-        }
-        red_release_add(X.sync + SYNC_ARRIVE, 1u);
-        const uint32_t target = (phase + 1) * (uint32_t)G;
-        if (ld_acquire(X.sync + SYNC_ARRIVE) < target) {
-            const uint64_t t0 = globaltimer();
-            for (uint32_t spin = 1;; ++spin) {
-                if (ld_acquire(X.sync + SYNC_ARRIVE) >= target) break;
+        for (int q = 0; q <= NWARPS; ++q) p += S.red[q][tid];
+        st_packet_relaxed(slot + (size_t)X.rank * PACKET_STRIDE + 2 * tid, p, tag);
+    }
+    const int nch = (X.G + 31) >> 5;  // chunks of a value
+    for (int ch = w; ch < NV * nch; ch += NWARPS + 1) {
+        const int k = ch / nch, c = (ch - k * nch) * 32 + lane;
+        __syncwarp();
+        double a = 0.0;
+        if (c < X.G) {
+            const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * k;
+            uint64_t t0 = 0;
+            for (uint32_t spin = 1; ld_packet_relaxed(pk, a) != tag; ++spin) {
                 if ((spin & 63u) == 0) {
+                    if (t0 == 0) t0 = globaltimer();
                     if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
                         S.abort = 1;
                         break;
@@ -722,27 +739,19 @@ __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (
                 }
             }
         }
+        __syncwarp();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) S.chunk[ch] = a;
     }
     __syncthreads();
     if (S.abort) return false;
-    if (w == 0) {
-        double a[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) a[k] = 0.0;
-        for (int c = lane; c < G; c += 32)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) a[k] += __ldcg(&X.partial[((size_t)slot * G + c) * 4 + k]);
-#pragma unroll
-        for (int k = 0; k < NV; ++k)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
-        if (lane == 0)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) S.bres[k] = a[k];
+    for (int k = 0; k < NV; ++k) {
+        double a = S.chunk[k * nch];
+        for (int ch = 1; ch < nch; ++ch) a += S.chunk[k * nch + ch];
+        out[k] = a;
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) out[k] = S.bres[k];
     ++phase;
     return true;
 }
@@ -759,9 +768,9 @@ __device__ bool grid_sum(const KParams &P, Smem &S, const double (&v)[NV], doubl
 __device__ void publish_x(const Ctx &X, uint32_t ep) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
+        fence_acq_rel_gpu();
         fence_proxy_async_global();
-        st_release(X.sync + SYNC_FLAGS + X.rank * FLAG_STRIDE, ep);
+        st_relaxed(X.sync + SYNC_FLAGS + X.rank * FLAG_STRIDE, ep);
     }
 }
 __device__ void publish(const KParams &P, uint32_t ep) { publish_x(ctx_of(P), ep); }
@@ -2820,7 +2829,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ Smem S;
     __shared__ unsigned s_q;
-    __shared__ int s_rng[4];
+    __shared__ int s_rng[4];  // own rows lo, hi; halo ranks lo, hi
     KParams P0;  // only the fields kernel_setup reads
     P0.nlay = 0;
     P0.stage_stride = B.stage_stride;
@@ -2828,8 +2837,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
     kernel_setup(P0, S, 0);
     const int tid = threadIdx.x;
     const int grp = blockIdx.x / B.gs, rank = blockIdx.x % B.gs;
-    const Ctx X{B.gsync + (size_t)grp * B.gsync_words, B.gpartial + (size_t)grp * 8 * B.gs, B.gs, rank,
+    // the group and the system in shared memory: their pointers would take
+    // the registers of the SpMV loops
+    __shared__ Ctx X;
+    __shared__ SysDesc D;
+    __shared__ SpmvSrc L;
+    if (tid == 0)
+        X = Ctx{B.gsync + (size_t)grp * B.gsync_words, B.gpartial + (size_t)grp * partial_words(B.gs), B.gs, rank,
                 B.limit_ns};
+    __syncthreads();
     Pipe pp;
     uint32_t phase = 0, ep = 0;
     const uint64_t vpol = policy_evict_last();
@@ -2844,46 +2860,41 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
         const unsigned qi = (unsigned)o0[0];
         if (qi >= (unsigned)B.count) break;
         const int sys = B.order[qi];
-        const SysDesc D = B.sys[sys];
+        if (tid == 0) D = B.sys[sys];  // the group_sum above ended with a barrier
+        __syncthreads();
         const uint8_t *hsrc = D.head + (size_t)rank * STAGES * ISSUE_REC;
         for (int i = tid; i < STAGES * ISSUE_REC; i += NTHREADS) (&S.head[0][0][0])[i] = hsrc[i];
         if (tid == 0) {
-            s_rng[0] = D.cta_slab[rank + 1] - D.cta_slab[rank];
-            s_rng[1] = D.cta_rb[rank];
-            s_rng[2] = D.cta_rb[rank + 1];
-            s_rng[3] = 0;
+            L.slabs = D.slabs;
+            L.head = &S.head[0][0][0];
+            L.ns = D.cta_slab[rank + 1] - D.cta_slab[rank];
+            L.kind = D.kind;
+            L.site = 40;
+            L.resident_ok = 1;  // within this system's solve
+            L.x32 = 0;          // FP64 layouts
+            L.gt = D.gt;
+            s_rng[0] = 16 * D.cta_rb[rank];
+            s_rng[1] = 16 * D.cta_rb[rank + 1];
+            s_rng[2] = D.cta_dep[2 * rank];
+            s_rng[3] = D.cta_dep[2 * rank + 1];
             // the ring holds the previous system's slabs
             for (int k = 0; k < STAGES; ++k) S.res_tag[k] = 0;
         }
         __syncthreads();
-        const int dep_lo = D.cta_dep[2 * rank], dep_hi = D.cta_dep[2 * rank + 1];
-        SpmvSrc L;
-        L.slabs = D.slabs;
-        L.head = &S.head[0][0][0];
-        L.ns = s_rng[0];
-        L.kind = D.kind;
-        L.site = 40;
-        L.resident_ok = 1;  // within this system's solve
-        L.x32 = 0;  // FP64 layouts
-        L.gt = D.gt;
-        const int vlo = s_rng[1] * 16, vhi = s_rng[2] * 16;
-        __syncthreads();  // s_rng read by all before the next system overwrites it
-        double *x = D.x, *r = D.r, *d = D.d, *q = D.q;
-        const double *b = D.b;
         // r = b - A x0, d = r (x0 is written before the launch: no halo wait)
-        EpiResidual er{b, r, 0.0, vpol};
-        if (!cta_spmv_src<false, EpiResidual, 8>(L, C, x, S, dyn, pp, er)) return;
+        EpiResidual er{D.b, D.r, 0.0, vpol};
+        if (!cta_spmv_src<false, EpiResidual, 8>(L, C, D.x, S, dyn, pp, er)) return;
         double bbp = 0.0;
-        MF_PAIRS(4, vlo, vhi, {
+        MF_PAIRS(4, s_rng[0], s_rng[1], {
             double2 rv[_vb], bv[_vb];
 #pragma unroll
-            MF_FOR_VB if (MF_LIVE(u, vhi)) {
-                rv[u] = ld2_hint(r + 2 * MF_PI(u), vpol);
-                bv[u] = ld2_hint(b + 2 * MF_PI(u), vpol);
+            MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
+                rv[u] = ld2_hint(D.r + 2 * MF_PI(u), vpol);
+                bv[u] = ld2_hint(D.b + 2 * MF_PI(u), vpol);
             }
 #pragma unroll
-            MF_FOR_VB if (MF_LIVE(u, vhi)) {
-                st2_hint(d + 2 * MF_PI(u), rv[u], vpol);
+            MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
+                st2_hint(D.d + 2 * MF_PI(u), rv[u], vpol);
                 bbp += bv[u].x * bv[u].x + bv[u].y * bv[u].y;
             }
         })
@@ -2896,9 +2907,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
         double rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
         int it = 0, status = MF_OK;
         while (it < maxit && (fixed || rel > B.tol)) {
-            if (!wait_deps_x(X, S, dep_lo, dep_hi, ep)) return;
-            EpiQ eq{d, q, 0.0, vpol};
-            if (!cta_spmv_src<false, EpiQ, 8>(L, C, d, S, dyn, pp, eq)) return;
+            if (!wait_deps_x(X, S, s_rng[2], s_rng[3], ep)) return;
+            EpiQ eq{D.d, D.q, 0.0, vpol};
+            if (!cta_spmv_src<false, EpiQ, 8>(L, C, D.d, S, dyn, pp, eq)) return;
             double v1[1] = {eq.dq}, o1[1];
             if (!group_sum<1>(X, S, v1, o1, phase)) return;
             const double dq = o1[0];
@@ -2908,19 +2919,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
             }
             const double alpha = rr / dq;
             double rrp = 0.0;
-            MF_PAIRS(4, vlo, vhi, {
+            MF_PAIRS(4, s_rng[0], s_rng[1], {
                 double2 rv[_vb], qv[_vb];
 #pragma unroll
-                MF_FOR_VB if (MF_LIVE(u, vhi)) {
-                    rv[u] = ld2_hint(r + 2 * MF_PI(u), vpol);
-                    qv[u] = ld2_hint(q + 2 * MF_PI(u), vpol);
+                MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
+                    rv[u] = ld2_hint(D.r + 2 * MF_PI(u), vpol);
+                    qv[u] = ld2_hint(D.q + 2 * MF_PI(u), vpol);
                 }
 #pragma unroll
-                MF_FOR_VB if (MF_LIVE(u, vhi)) {
+                MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
                     double2 o;
                     o.x = rv[u].x - alpha * qv[u].x;
                     o.y = rv[u].y - alpha * qv[u].y;
-                    st2_hint(r + 2 * MF_PI(u), o, vpol);
+                    st2_hint(D.r + 2 * MF_PI(u), o, vpol);
                     rrp += o.x * o.x + o.y * o.y;
                 }
             })
@@ -2931,24 +2942,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
             rel = bnorm > 0 ? sqrt(rrn) / bnorm : 0.0;
             const double beta = rrn / rr;
             const bool done = !fixed && rel <= B.tol;
-            MF_PAIRS(4, vlo, vhi, {
+            MF_PAIRS(4, s_rng[0], s_rng[1], {
                 double2 dv[_vb], xv[_vb], rv[_vb];
 #pragma unroll
-                MF_FOR_VB if (MF_LIVE(u, vhi)) {
-                    dv[u] = ld2_hint(d + 2 * MF_PI(u), vpol);
-                    xv[u] = ld2_hint(x + 2 * MF_PI(u), vpol);
-                    rv[u] = ld2_hint(r + 2 * MF_PI(u), vpol);
+                MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
+                    dv[u] = ld2_hint(D.d + 2 * MF_PI(u), vpol);
+                    xv[u] = ld2_hint(D.x + 2 * MF_PI(u), vpol);
+                    rv[u] = ld2_hint(D.r + 2 * MF_PI(u), vpol);
                 }
 #pragma unroll
-                MF_FOR_VB if (MF_LIVE(u, vhi)) {
+                MF_FOR_VB if (MF_LIVE(u, s_rng[1])) {
                     double2 xo, dn;
                     xo.x = xv[u].x + alpha * dv[u].x;
                     xo.y = xv[u].y + alpha * dv[u].y;
-                    st2_hint(x + 2 * MF_PI(u), xo, vpol);
+                    st2_hint(D.x + 2 * MF_PI(u), xo, vpol);
                     if (!done) {
                         dn.x = rv[u].x + beta * dv[u].x;
                         dn.y = rv[u].y + beta * dv[u].y;
-                        st2_hint(d + 2 * MF_PI(u), dn, vpol);
+                        st2_hint(D.d + 2 * MF_PI(u), dn, vpol);
                     }
                 }
             })
@@ -3004,6 +3015,7 @@ int kernel_config(mf_tiles *t, int *G_out) {
     int per_sm = t->opt.ctas_per_sm > 0 ? t->opt.ctas_per_sm : 1;
     if (per_sm > occ_min) per_sm = occ_min;
     *G_out = t->nsm * per_sm;
+    if (*G_out > 32 * MAX_CHUNKS) *G_out = 32 * MAX_CHUNKS;  // group_sum's chunk sums
     return MF_OK;
 }
 

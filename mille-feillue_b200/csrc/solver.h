@@ -14,7 +14,13 @@ constexpr int PRODUCER_WARP = NWARPS;      // one more warp issues the bulk copi
 constexpr int NTHREADS = (NWARPS + 1) * 32;
 constexpr int KMAX_LAYOUTS = 1 + MF_NLEVELS;
 constexpr int FLAG_STRIDE = 8;             // one 32-byte sector per CTA flag
-enum { SYNC_ARRIVE = 0, SYNC_ERROR = 32, SYNC_SITE = 33, SYNC_FLAGS = 64 };
+enum { SYNC_ERROR = 32, SYNC_SITE = 33, SYNC_FLAGS = 64 };
+// Doubles of the reduction packets of G CTAs (zero before each launch): 2
+// slots x G CTAs x PACKET_STRIDE doubles (a 128-byte line), of which
+// PACKET_VALUES {value, phase tag} pairs are used.
+constexpr int PACKET_VALUES = 4, PACKET_STRIDE = 16;
+constexpr int MAX_CHUNKS = 32;  // of 32 CTAs: grids of up to 1024 CTAs
+__host__ __device__ inline size_t partial_words(int G) { return 2 * PACKET_STRIDE * (size_t)G; }
 inline size_t sync_words(int G) { return (size_t)SYNC_FLAGS + (size_t)G * FLAG_STRIDE + 32; }
 
 inline int slab_area_of(int slab_max) { return (slab_max + 127) & ~127; }
@@ -91,8 +97,8 @@ struct BatchParams {
     int stage_stride, slab_area;
     uint64_t limit_ns;
     int gs, gsync_words;  // CTAs per group; sync words per group
-    uint32_t *gsync;      // per group: arrive counter, error word, rank flags
-    double *gpartial;     // per group: 2 slots x gs x 4 partial sums
+    uint32_t *gsync;      // per group: error word, rank flags
+    double *gpartial;     // per group: partial_words(gs), zero before the launch
     BatchResult *res;
 };
 int launch_batch(const BatchParams &B, int grid, cudaStream_t s);

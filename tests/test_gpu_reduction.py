@@ -1,0 +1,32 @@
+"""The group-wide sums of the persistent solvers (one packet per CTA, polled
+32 CTAs a warp) at the edges of their chunks: groups of 1, 31, 32, 33, 65 and
+all 148 CTAs, through the batched CG, whose group size is an option."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("gs", [1, 31, 32, 33, 65, 148])
+def test_group_sums_at_chunk_edges(mf, O, gs):
+    import scipy.sparse as sp
+    import torch
+
+    mats = [mf.Matrix.spd_random(n, 40 + n) for n in (33, 5000)] + [mf.Matrix.poisson2d(37)]
+    o = mf.options()
+    o.reserved[4] = gs
+    B = mf.Batch(mats, o)
+    b = torch.tensor(np.concatenate([m.b() for m in mats]), device="cuda")
+    x = torch.zeros_like(b)
+    for _ in range(2):  # the second solve starts from the first one's packets
+        B.solve_cg_dev(b.data_ptr(), x.data_ptr(), 1e-10, 10000)
+    it, st, rel = B.results()
+    assert np.all(st == 0) and np.all(rel <= 1e-10)
+    xh = x.cpu().numpy()
+    for s, m in enumerate(mats):
+        rp, ci, v = m.csr()
+        M = sp.csr_matrix((v, ci, rp), shape=(m.n, m.n))
+        xs = xh[B.offsets[s]:B.offsets[s + 1]]
+        assert np.linalg.norm(m.b() - M @ xs) / np.linalg.norm(m.b()) <= 1.5e-10
+        it_o, _, _ = O.OracleTiles(m.n, m.n, rp, ci, v).cg(m.b(), 1e-10, 10000)
+        assert abs(int(it[s]) - it_o) <= max(2, 0.02 * it_o), (s, it[s], it_o)
