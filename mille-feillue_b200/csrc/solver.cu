@@ -60,22 +60,6 @@ __device__ void set_error_w(uint32_t *sync, uint32_t code, uint32_t site) {
 }
 __device__ void set_error(const KParams &P, uint32_t code, uint32_t site) { set_error_w(P.sync, code, site); }
 
-// Thread 0: issue the bulk copies of one slab (x runs first, slab last: the
-// issue record may live inside the stage the slab overwrites).
-// An x segment is 16 entries: 128 bytes of FP64 x, 64 bytes of FP32 x.
-__device__ void issue_slab(Smem &S, uint8_t *stage, int xoff, int k, uint32_t off16, uint32_t bytes,
-                           uint32_t xbytes, int nruns, const XRun *runs, const uint8_t *slabs,
-                           const uint8_t *xv, uint32_t segb, uint64_t pol_m, uint64_t pol_v) {
-    mbar_arrive_expect_tx(&S.full[k], bytes + xbytes);
-    uint8_t *xarea = stage + xoff;
-    for (int q = 0; q < nruns; ++q) {
-        const XRun r = runs[q];
-        bulk_g2s(xarea + (size_t)r.slot0 * segb, xv + (size_t)r.seg0 * segb, (uint32_t)r.nseg * segb, &S.full[k],
-                 pol_v);
-    }
-    bulk_g2s(stage, slabs + (size_t)off16 * 16, bytes, &S.full[k], pol_m);
-}
-
 // Pipeline state kept in registers across SpMV calls: consumer parity of
 // each stage's full barrier, producer parity of each stage's empty barrier,
 // and the stages filled at least once (whose refill must wait for empty).
@@ -487,9 +471,9 @@ __device__ double global_row(const GTiles &P, int rb, int r, const double *__res
 }
 
 // Tiled SpMV of this CTA's row range with layout `lay` and input vector xv.
-// Warp PRODUCER_WARP (one lane) streams the CTA's slabs into the STAGES-deep
-// ring: it waits until the consumers released a stage, then issues the x
-// runs and the slab of the next slab with 1D bulk copies. The NWARPS
+// Warp PRODUCER_WARP streams the CTA's slabs into the STAGES-deep ring: it
+// waits until the consumers released a stage, then issues the slab and the x
+// runs of the next slab with 1D bulk copies. The NWARPS
 // consumer warps wait for a stage's full barrier, compute their row blocks
 // (one half-warp per row block, one lane per row) and release the stage.
 // For every row < rowA: v = epi.pre(row) (any type) is loaded before the row's
@@ -505,62 +489,69 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
     const int w = tid >> 5, lane = tid & 31;
     const int half = lane >> 4, r = lane & 15;
     if (w == PRODUCER_WARP) {
-        if (lane == 0) {
-            const uint64_t pm = policy_evict_first(), pv = policy_evict_last();
-            fence_proxy_async_global();
-            for (int i = 0; i < ns; ++i) {
-                const int k = i % STAGES;
-                uint8_t *st = stage_ptr(dyn, k, stride);
-                if ((pp.filled >> k) & 1u) {
-                    if (!wait_bar(&S.empty[k], (pp.eph >> k) & 1u, C.limit_ns)) {
-                        set_error_w(C.sync, (uint32_t)MF_ERR_TIMEOUT, 110 + L.site);
-                        S.abort = 1;
-                        break;
-                    }
-                    pp.eph ^= 1u << k;
+        // The whole warp issues: lane q the copy of x run q (MAXRUNS <= 32),
+        // lane 0 the slab. One lane reading and issuing ~20 runs in turn kept
+        // the first slab of a CTA waiting, which every SpMV of a solve pays:
+        // 5-point 256^2 1.73 -> 1.47 us, 7-point 75^3 7.1 -> 6.7 us, 128^3
+        // standalone 27.4 -> 26.9 us.
+        const uint64_t pm = policy_evict_first(), pv = policy_evict_last();
+        const uint32_t segb = L.x32 ? 64u : 128u;  // an x segment: 16 entries
+        fence_proxy_async_global();
+        for (int i = 0; i < ns; ++i) {
+            const int k = i % STAGES;
+            uint8_t *st = stage_ptr(dyn, k, stride);
+            if ((pp.filled >> k) & 1u) {
+                if (!wait_bar(&S.empty[k], (pp.eph >> k) & 1u, C.limit_ns)) {
+                    set_error_w(C.sync, (uint32_t)MF_ERR_TIMEOUT, 110 + L.site);
+                    S.abort = 1;
+                    break;
                 }
-                pp.filled |= 1u << k;
-                uint32_t off16, bytes, xbytes;
-                int nruns;
-                const XRun *runs;
-                if (i < STAGES) {
-                    const uint32_t *rec = reinterpret_cast<const uint32_t *>(L.head + i * ISSUE_REC);
-                    off16 = rec[0];
-                    bytes = rec[1];
-                    xbytes = rec[2];
-                    nruns = (int)rec[3];
-                    runs = reinterpret_cast<const XRun *>(rec + 4);
-                } else {
-                    // the slab consumed from this stage carries the record of slab i
-                    const SlabHeader *h = reinterpret_cast<const SlabHeader *>(st);
-                    off16 = h->next_off16;
-                    bytes = h->next_bytes;
-                    xbytes = h->next_xbytes;
-                    nruns = h->next_nruns;
-                    runs = reinterpret_cast<const XRun *>(st + SLAB_HDR);
-                    if (C.prefetch && h->pf_bytes) bulk_prefetch_l2(L.slabs + (size_t)h->pf_off16 * 16, h->pf_bytes);
-                }
-                fence_proxy_async_smem();
-                // a CTA with at most STAGES slabs puts slab i in stage i on
-                // every SpMV: when the stage still holds it (same layout,
-                // nothing else written into the ring since), only its x
-                // window is copied
-                const bool keep = L.resident_ok && ns <= STAGES;
-                if (keep && S.res_tag[k] == (uint8_t)(L.site + 1)) {
-                    mbar_arrive_expect_tx(&S.full[k], xbytes);
-                    const uint32_t segb = L.x32 ? 64u : 128u;
-                    for (int q = 0; q < nruns; ++q) {
-                        const XRun rr = runs[q];
-                        bulk_g2s(st + xoff + (size_t)rr.slot0 * segb,
-                                 static_cast<const uint8_t *>(xv) + (size_t)rr.seg0 * segb, (uint32_t)rr.nseg * segb,
-                                 &S.full[k], pv);
-                    }
-                } else {
-                    issue_slab(S, st, xoff, k, off16, bytes, xbytes, nruns, runs, L.slabs,
-                               static_cast<const uint8_t *>(xv), L.x32 ? 64u : 128u, pm, pv);
+                pp.eph ^= 1u << k;
+            }
+            pp.filled |= 1u << k;
+            uint32_t off16, bytes, xbytes;
+            int nruns;
+            const XRun *runs;
+            if (i < STAGES) {
+                const uint32_t *rec = reinterpret_cast<const uint32_t *>(L.head + i * ISSUE_REC);
+                off16 = rec[0];
+                bytes = rec[1];
+                xbytes = rec[2];
+                nruns = (int)rec[3];
+                runs = reinterpret_cast<const XRun *>(rec + 4);
+            } else {
+                // the slab consumed from this stage carries the record of slab i
+                const SlabHeader *h = reinterpret_cast<const SlabHeader *>(st);
+                off16 = h->next_off16;
+                bytes = h->next_bytes;
+                xbytes = h->next_xbytes;
+                nruns = h->next_nruns;
+                runs = reinterpret_cast<const XRun *>(st + SLAB_HDR);
+                if (C.prefetch && lane == 0 && h->pf_bytes)
+                    bulk_prefetch_l2(L.slabs + (size_t)h->pf_off16 * 16, h->pf_bytes);
+            }
+            XRun run = {0, 0, 0};
+            if (lane < nruns) run = runs[lane];
+            // a CTA with at most STAGES slabs puts slab i in stage i on
+            // every SpMV: when the stage still holds it (same layout,
+            // nothing else written into the ring since), only its x
+            // window is copied
+            const bool keep = L.resident_ok && ns <= STAGES;
+            const bool held = keep && S.res_tag[k] == (uint8_t)(L.site + 1);
+            fence_proxy_async_smem();
+            __syncwarp();  // the record is read before the slab lands on it
+            if (lane == 0) {
+                mbar_arrive_expect_tx(&S.full[k], held ? xbytes : bytes + xbytes);
+                if (!held) {
+                    bulk_g2s(st, L.slabs + (size_t)off16 * 16, bytes, &S.full[k], pm);
                     S.res_tag[k] = keep ? (uint8_t)(L.site + 1) : (uint8_t)0;
                 }
             }
+            __syncwarp();  // expected before any lane's copy can complete
+            if (lane < nruns)
+                bulk_g2s(st + xoff + (size_t)run.slot0 * segb,
+                         static_cast<const uint8_t *>(xv) + (size_t)run.seg0 * segb, (uint32_t)run.nseg * segb,
+                         &S.full[k], pv);
         }
         __syncwarp();
     } else {
