@@ -11,7 +11,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "solver.h"
@@ -59,17 +61,54 @@ struct mf_batch {
 
 namespace {
 
-constexpr int kBatchGroupDefault = 4;  // CTAs per system group (fastest of 4, 8, 16 on the 512-system set)
+constexpr int kBatchGroupMin = 4;  // smallest group the rule below considers
+
+// CTAs per group when the caller leaves the choice: the group size whose
+// launch ends first when the systems, largest first, go to whichever group
+// is free. One iteration of a system on gs CTAs takes about kIterUs plus
+// kNnzUs * nnz / gs (scattered systems, whose gathers bound them; equal
+// iteration counts). Small groups keep every CTA busy when there are many
+// systems (512 of 1e3..2e5 rows: 4 CTAs); with few, the largest system alone
+// would hold the launch (48 such systems: 74.2 ms in groups of 4, 21.2 in 16,
+// 26.1 in 37, 22.2 in the chosen 13; 3 systems: 32.5 ms in 4, 4.3 in 37, 2.7
+// in the chosen 148).
+constexpr double kIterUs = 10.0, kNnzUs = 1.1e-3;
+int choose_group(int nsm, std::vector<long long> nnz) {
+    std::sort(nnz.begin(), nnz.end(), std::greater<long long>());
+    int best = nsm < kBatchGroupMin ? nsm : kBatchGroupMin;
+    double best_us = 1e300;
+    for (int ng = std::max(1, nsm / kBatchGroupMin), last = 0; ng >= 1; --ng) {
+        const int gs = nsm / ng;
+        if (gs == last) continue;
+        last = gs;
+        std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+        for (int g = 0; g < ng; ++g) free_at.push(0.0);
+        double end = 0.0;
+        for (long long z : nnz) {
+            const double t = free_at.top() + kIterUs + kNnzUs * (double)z / gs;
+            free_at.pop();
+            free_at.push(t);
+            end = std::max(end, t);
+        }
+        if (end < best_us) {
+            best_us = end;
+            best = gs;
+        }
+    }
+    return best;
+}
 // group sync words: error word, rank flags (32-byte aligned)
 size_t group_sync_words(int gs) { return (sync_words(gs) + 7) & ~(size_t)7; }
 
-// packed[poff_s + i] <-> ws vector of system s, row i (i < n_s)
+// packed[poff_s + i] <-> ws vector of system s, row i (i < n_s); kCopyY
+// blocks share a system (one block took 0.3 ms for 2e5 rows)
+constexpr int kCopyY = 32;
 __global__ void k_scatter(const double *packed, double *ws, const long long *voff, const long long *poff,
                           const int *n, int count, long long ws_rows, int which) {
     for (int s = blockIdx.x; s < count; s += gridDim.x) {
         double *dst = ws + (long long)which * ws_rows + voff[s];
         const double *src = packed + poff[s];
-        for (int i = threadIdx.x; i < n[s]; i += blockDim.x) dst[i] = src[i];
+        for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n[s]; i += gridDim.y * blockDim.x) dst[i] = src[i];
     }
 }
 __global__ void k_gather(double *packed, const double *ws, const long long *voff, const long long *poff,
@@ -77,7 +116,7 @@ __global__ void k_gather(double *packed, const double *ws, const long long *voff
     for (int s = blockIdx.x; s < count; s += gridDim.x) {
         const double *src = ws + (long long)which * ws_rows + voff[s];
         double *dst = packed + poff[s];
-        for (int i = threadIdx.x; i < n[s]; i += blockDim.x) dst[i] = src[i];
+        for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < n[s]; i += gridDim.y * blockDim.x) dst[i] = src[i];
     }
 }
 
@@ -120,7 +159,7 @@ int mf_batch_create(int count, const mf_csr *systems, const mf_options *opt_in, 
     {
         int nsm = 0;
         MF_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, opt.device));
-        int gs = opt.reserved[4] > 0 ? opt.reserved[4] : kBatchGroupDefault;
+        int gs = opt.reserved[4] > 0 ? opt.reserved[4] : choose_group(nsm, B->nnz);
         if (gs > nsm) gs = nsm;
         B->gs = gs;
         B->ngroups = nsm / gs;
@@ -231,7 +270,7 @@ int mf_batch_solve_cg_dev(mf_batch *B, const double *b, double *x, double tol, i
         cudaMemsetAsync(B->d_sync.p, 0, sizeof(uint32_t) * B->d_sync.n, s);
         cudaMemsetAsync(B->d_partial.p, 0, sizeof(double) * B->d_partial.n, s);  // the packets' phase tags
         cudaMemsetAsync(B->ws.p, 0, sizeof(double) * 5 * B->ws_rows, s);
-        k_scatter<<<std::min(B->count, 1024), 256, 0, s>>>(b, B->ws.p, B->d_voff.p, B->d_poff.p, B->d_n.p,
+        k_scatter<<<dim3(std::min(B->count, 1024), kCopyY), 256, 0, s>>>(b, B->ws.p, B->d_voff.p, B->d_poff.p, B->d_n.p,
                                                           B->count, B->ws_rows, 0);
         const int lrc = launch_batch(P, B->grid, s);
         if (lrc) {
@@ -240,7 +279,7 @@ int mf_batch_solve_cg_dev(mf_batch *B, const double *b, double *x, double tol, i
             if (g) cudaGraphDestroy(g);
             return lrc;
         }
-        k_gather<<<std::min(B->count, 1024), 256, 0, s>>>(x, B->ws.p, B->d_voff.p, B->d_poff.p, B->d_n.p,
+        k_gather<<<dim3(std::min(B->count, 1024), kCopyY), 256, 0, s>>>(x, B->ws.p, B->d_voff.p, B->d_poff.p, B->d_n.p,
                                                          B->count, B->ws_rows, 1);
         MF_CUDA_TRY(cudaStreamEndCapture(s, &B->graph));
         MF_CUDA_TRY(cudaGraphInstantiate(&B->gexec, B->graph, 0));
