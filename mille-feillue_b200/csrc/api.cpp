@@ -84,11 +84,13 @@ int ensure_host_tiles(const mf_tiles *t) {
 }
 
 // Encodes a device CSR; G > 0 forces the number of CTA ranges of the layout
-// (1 for the batched solver, whose CTAs each own a whole system).
+// (the CTAs of a group, for the batched solver), all_gather a layout in gather
+// mode only.
 int encode_dev_impl(int n, int ncols, int nnz, const int *rp, const int *ci, const double *val,
-                    const mf_options *opt, int G_force, mf_tiles **out) {
+                    const mf_options *opt, int G_force, bool all_gather, mf_tiles **out) {
     if (!out || n <= 0 || ncols <= 0 || nnz < 0 || !rp || (nnz > 0 && (!ci || !val))) return MF_ERR_ARG;
     auto *t = new mf_tiles;
+    t->all_gather = all_gather;
     if (opt) t->opt = *opt;
     else mf_options_default(&t->opt);
     int rc;
@@ -113,7 +115,7 @@ extern "C" {
 
 int mf_encode_dev(int n, int ncols, int nnz, const int *rp, const int *ci, const double *val,
                   const mf_options *opt, mf_tiles **out) {
-    return mf::encode_dev_impl(n, ncols, nnz, rp, ci, val, opt, 0, out);
+    return mf::encode_dev_impl(n, ncols, nnz, rp, ci, val, opt, 0, false, out);
 }
 
 int mf_encode(const mf_csr *A, const mf_options *opt, mf_tiles **out) {
@@ -162,7 +164,7 @@ double dev_bytes(const DevArray<T> &a) {
 }
 double layout_dev_bytes(const Layout &L) {
     return dev_bytes(L.slabs) + dev_bytes(L.head) + dev_bytes(L.cta_slab) + dev_bytes(L.cta_rb) +
-           dev_bytes(L.cta_dep) + dev_bytes(L.prec_dev) + dev_bytes(L.scale_dev);
+           dev_bytes(L.cta_dep) + dev_bytes(L.rbtab) + dev_bytes(L.prec_dev) + dev_bytes(L.scale_dev);
 }
 }  // namespace
 }  // extern "C++"
@@ -537,7 +539,7 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     // holds the vector passes' copies, and one CTA runs per SM (each CTA
     // allocates all of the SM's tensor memory)
     if ((launch_kind == 2 || launch_kind == 4 || (launch_kind == 0 && !mixed)) && opt.reserved[5] != 1 &&
-        t->G == t->nsm) {
+        t->G == t->nsm && !(launch_kind == 0 && t->L64.direct)) {
         int rows_max = 0;
         for (size_t g = 0; g + 1 < t->h_cta_rb.size(); ++g)
             rows_max = std::max(rows_max, 16 * (t->h_cta_rb[g + 1] - t->h_cta_rb[g]));

@@ -157,6 +157,18 @@ MF_DEV void stf_hint(float *p, float v, uint64_t pol) {
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(pol) : "memory");
 }
 
+// Constant data read once a pass, a warp's lanes side by side: past L1.
+MF_DEV uint32_t ld_stream(const uint32_t *p) {
+    uint32_t v;
+    asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+MF_DEV double ld_stream(const double *p) {
+    double v;
+    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 // ---- tensor memory (TMEM): 128 lanes x 512 columns of 32 bits per SM.
 // Allocation and release are whole-warp operations; a warp of a warpgroup
 // reaches lanes 32*(warp % 4) .. +31 only. taddr = lane << 16 | column.

@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(FILL_THREADS) k_fill_slabs(const SlabPlan *__r
                                                              const int *__restrict__ rbW,
                                                              const unsigned *__restrict__ rbvb,
                                                              const uint8_t *__restrict__ rbaff, bool mixed,
-                                                             uint32_t segbytes, uint32_t zpos, uint8_t *slabs) {
+                                                             uint32_t segbytes, uint32_t zpos, uint8_t *slabs,
+                                                             RbEntry *rbtab) {
     __shared__ uint32_t s_off[RB_PER_SLAB_MAX + 1];
     const int s = blockIdx.x;
     const SlabPlan P = plans[s];
@@ -348,6 +349,7 @@ __global__ void __launch_bounds__(FILL_THREADS) k_fill_slabs(const SlabPlan *__r
                 s_off[j] = off;
                 const int W = rbW[P.rb0 + j];
                 dir[j].off = off;
+                if (rbtab) rbtab[P.rb0 + j] = RbEntry{P.off16 + off / 16u, (uint32_t)W};
                 uint32_t dslot = 0;  // own column segment in the staged x window
                 if (P.mode == SLAB_STAGED) {
                     const int *sg = segs + P.seg_off;
@@ -1024,7 +1026,7 @@ int build_layout(mf_tiles *t, Layout &L, const std::vector<uint8_t> &prec_in, cu
     uint64_t off = 0;
     int ns = 0, nsegs = 0, nruns = 0;
     for (;;) {
-        xseg_max = x32 ? xseg_max32(slab_area) : XSEG_MAX;
+        xseg_max = x32 ? xseg_max32(slab_area) : (t->all_gather && !mixed) ? -1 : XSEG_MAX;
         segbytes = x32 ? 64u : 128u;
         rbps = t->opt.rb_per_slab > 0 ? std::min(t->opt.rb_per_slab, RB_PER_SLAB_MAX)
                                       : (x32 ? RB_PER_SLAB_X32 : RB_PER_SLAB_X64);
@@ -1146,10 +1148,14 @@ int build_layout(mf_tiles *t, Layout &L, const std::vector<uint8_t> &prec_in, cu
     if (L.slabs.alloc(off + 16) || L.cta_rb.alloc(G + 1) || L.cta_dep.alloc(2 * G)) return MF_ERR_NOMEM;
     MF_CUDA_TRY(cudaMemcpyAsync(L.cta_rb.p, cta_rb.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, st));
     MF_CUDA_TRY(cudaMemcpyAsync(L.cta_dep.p, dep.data(), sizeof(int) * 2 * G, cudaMemcpyHostToDevice, st));
+    // direct: no row block staged or oversize (empty row blocks count as
+    // staged, with no segments)
+    const bool direct = !mixed && ns > 0 && n_over == 0 && nsegs == 0;
+    if (direct && L.rbtab.alloc(tilem)) return MF_ERR_NOMEM;
     if (ns > 0)
         k_fill_slabs<<<ns, FILL_THREADS, 0, st>>>(d_plans.p, d_slab_cta.p, L.cta_slab.p, d_segs.p, d_runs.p, A,
                                                  d_rbW.p, d_rbvb.p, d_rbaff.p, mixed, segbytes,
-                                                 zero_pos_of(slab_area, x32), L.slabs.p);
+                                                 zero_pos_of(slab_area, x32), L.slabs.p, direct ? L.rbtab.p : nullptr);
     MF_CUDA_TRY(cudaGetLastError());
     MF_CUDA_TRY(cudaStreamSynchronize(st));
     L.prec.swap(prec);
@@ -1162,6 +1168,7 @@ int build_layout(mf_tiles *t, Layout &L, const std::vector<uint8_t> &prec_in, cu
     L.mixed = mixed;
     L.kind = kind;
     L.x32 = x32;
+    L.direct = direct;
     L.bytes = off;
     L.alg_bytes = alg;
     for (int p = 0; p < 4; ++p) L.tile_frac[p] = tilenum > 0 ? cnt[p] / tilenum : 0.0;

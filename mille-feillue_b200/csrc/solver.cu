@@ -29,8 +29,10 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 #include "solver.h"
@@ -643,10 +645,120 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
 }
 
 
+constexpr int DIRECT_GB = 8;  // gathers of x a lane keeps in flight
+
+// Rows r of the gather blocks rb, rb + step, ... < hi of a direct layout, one
+// lane a row, in blockspmv_cpu's order (as slab_row): fin(rb, row sum) for
+// each. GB gathers of x a lane are in flight; meanwhile the indices and
+// values of the next GB planes, of the next row block where this one ends,
+// and the table entry of the one after it are loaded. x through L1: the halo
+// wait before the SpMV is an acquire, after which no older line of it is read.
+template <int GB, class Pre, class Fin>
+__device__ __forceinline__ void gather_rows(const uint8_t *slabs, const RbEntry *rbtab, int rb, int step, int hi,
+                                            int r, const double *xg, Pre pre, Fin fin) {
+    if (rb >= hi) return;
+    auto entry = [&](int j) { return j < hi ? __ldg(reinterpret_cast<const uint2 *>(rbtab + j)) : make_uint2(0u, 1u); };
+    uint2 e = entry(rb), en = entry(rb + step);
+    auto idx_of = [&](uint2 q) { return reinterpret_cast<const uint32_t *>(slabs + (size_t)q.x * 16 + rb_idx_off()) + r; };
+    auto val_of = [&](uint2 q) {
+        return reinterpret_cast<const double *>(slabs + (size_t)q.x * 16 + rb_vals_off((int)q.y, true)) + r;
+    };
+    uint32_t id[GB];
+    double v[GB];
+    const uint32_t *ip = idx_of(e);
+    const double *vp = val_of(e);
+    int left = (int)e.y;  // planes of this row block from the current ones on
+#pragma unroll
+    for (int u = 0; u < GB; ++u) {
+        const int q = left > 0 ? min(u, left - 1) : 0;
+        id[u] = left > 0 ? ld_stream(ip + 16 * q) : IDX32_PAD;
+        v[u] = left > 0 ? ld_stream(vp + 16 * q) : 0.0;
+        if (u >= left) id[u] = IDX32_PAD;
+    }
+    double acc = 0.0, sum = 0.0;
+    auto pv = pre(rb);
+#pragma unroll 1
+    while (true) {
+        double x[GB];
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            x[u] = 0.0;
+            if (!(id[u] & IDX32_PAD)) x[u] = xg[id[u] & IDX32_POS];
+        }
+        const bool last = left <= GB;  // the row block's last planes
+        const int rbn = last ? rb + step : rb;
+        uint2 ef = en;
+        if (last) {
+            ip = idx_of(en);
+            vp = val_of(en);
+            left = rbn < hi ? (int)en.y : 0;
+            ef = entry(rbn + step);
+        } else {
+            ip += 16 * GB;
+            vp += 16 * GB;
+            left -= GB;
+        }
+        uint32_t nid[GB];
+        double nv[GB];
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            const int q = left > 0 ? min(u, left - 1) : 0;
+            nid[u] = left > 0 ? ld_stream(ip + 16 * q) : IDX32_PAD;
+            nv[u] = left > 0 ? ld_stream(vp + 16 * q) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            if (id[u] & IDX32_START) {
+                acc = dadd(acc, sum);
+                sum = 0.0;
+            }
+            if (!(id[u] & IDX32_PAD)) sum = dadd(sum, dmul(x[u], v[u]));
+            id[u] = u < left ? nid[u] : IDX32_PAD;
+            v[u] = nv[u];
+        }
+        if (last) {
+            fin(rb, dadd(acc, sum), pv);
+            if (rbn >= hi) return;
+            acc = sum = 0.0;
+            pv = pre(rbn);
+            rb = rbn;
+            en = ef;
+        }
+    }
+}
+
+// The SpMV of this CTA's row blocks [lo, hi) on a direct layout: one half-warp
+// a row block, every warp, no copy ring. Scattered columns make the gathers
+// of x the cost, and what hides their latency is row blocks in flight: a slab
+// of the ring holds about 7 row blocks of 17 entries a row, so 4 stages keep
+// at most 28 half-warps busy, and only while no stage is being refilled.
+// Random 8-byte gathers peak at 1.9 per ns and SM (measured; 12 us for 2e5
+// rows of 17 entries). CG on such a system: 45.2 us an iteration through the
+// ring, 34.2 here; 48 systems of 1e3..2e5 rows in one launch 22.1 -> 15.6 ms.
+template <int GB, class Epi>
+__device__ __forceinline__ void cta_spmv_direct(const uint8_t *slabs, const RbEntry *rbtab, int lo, int hi, int rowA,
+                                                const double *x, Epi &epi) {
+    const int r = threadIdx.x & 15;
+    using PV = decltype(epi.pre(0));
+    gather_rows<GB>(
+        slabs, rbtab, lo + (int)(threadIdx.x >> 4), NTHREADS / 16, hi, r, x,
+        [&](int rb) { return rb * 16 + r < rowA ? epi.pre(rb * 16 + r) : PV(0); },
+        [&](int rb, double acc, PV pv) {
+            if (rb * 16 + r < rowA) epi(rb * 16 + r, acc, pv);
+        });
+    __syncthreads();
+}
+
 // Grid-kernel form: layout `lay` of the kernel parameters, this CTA's slabs.
 // xv: FP64 vector, or FP32 when the layout stages x in FP32.
-template <bool MIXED, class Epi, int GB = 1>
+// DIRECT: the layout is direct.
+template <bool MIXED, bool DIRECT = false, int GB = 1, class Epi>
 __device__ bool cta_spmv(const KParams &P, int lay, const void *xv, Smem &S, uint8_t *dyn, Pipe &pp, Epi &epi) {
+    if constexpr (DIRECT) {
+        cta_spmv_direct<DIRECT_GB>(P.lay[lay].slabs, P.lay[lay].rbtab, P.lay[lay].cta_rb[blockIdx.x],
+                           P.lay[lay].cta_rb[blockIdx.x + 1], P.rowA, static_cast<const double *>(xv), epi);
+        return S.abort == 0;
+    }
     SpmvSrc L;
     L.slabs = P.lay[lay].slabs;
     L.head = &S.head[lay][0][0];
@@ -810,7 +922,7 @@ __device__ __forceinline__ void zero_slots(uint8_t *dyn, int stage_stride, int s
 __device__ void kernel_setup(const KParams &P, Smem &S, int nlay) {
     extern __shared__ __align__(128) uint8_t dyn[];
     const int tid = threadIdx.x;
-    zero_slots(dyn, P.stage_stride, P.slab_area);
+    if (P.stage_stride > 0) zero_slots(dyn, P.stage_stride, P.slab_area);  // 0: launched without a ring
     if (tid == 0) {
         for (int k = 0; k < STAGES; ++k) {
             mbar_init(&S.full[k], 1);
@@ -868,8 +980,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_spmv(KParams P, const void *x, 
     Pipe pp;
     EpiStore epi{y};
     for (int it = 0; it < reps; ++it) {
-        if (!cta_spmv<MIXED, EpiStore, 8>(P, lay, x, S, dyn, pp, epi)) return;
+        if (!cta_spmv<MIXED, false, 8>(P, lay, x, S, dyn, pp, epi)) return;
     }
+}
+
+// The standalone SpMV of a direct layout. 2e5 scattered rows of 17 entries:
+// 31.0 us through the copy ring, 21.5 here; 5000 rows 4.9 -> 3.3 us.
+constexpr int DIRECT_THREADS = 64, DIRECT_CTAS = 8;  // threads a CTA, CTAs an SM (small CTAs spread small systems)
+__global__ void __launch_bounds__(DIRECT_THREADS, DIRECT_CTAS)
+    k_spmv_direct(const uint8_t *slabs, const RbEntry *__restrict__ rbtab, int tilem, int rowA, const double *x,
+                  double *y) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int r = threadIdx.x & 15;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    gather_rows<DIRECT_GB>(
+        slabs, rbtab, blockIdx.x * (DIRECT_THREADS / 16) + (int)(threadIdx.x >> 4), gridDim.x * (DIRECT_THREADS / 16),
+        tilem, r, x, [](int) { return 0; },
+        [&](int rb, double acc, int) {
+            if (rb * 16 + r < rowA) y[rb * 16 + r] = acc;
+        });
 }
 
 // -------------------------------------------------------------------- CG
@@ -923,7 +1052,8 @@ struct EpiQ {  // q = A d, dq += d*q
             P.trace[(size_t)(it) * 8 + (s)] = globaltimer();                              \
     } while (0)
 
-template <bool MIXED>
+// DIRECT: the FP64 layout is direct (FP64 only).
+template <bool MIXED, bool DIRECT = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ Smem S;
@@ -946,7 +1076,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
     }
     // r = b - A x0, d = r; (rr, bb)
     EpiResidual er{b, r, 0.0, vpol};
-    if (!cta_spmv<false>(P, lay64, x, S, dyn, pp, er)) return;
+    if (!cta_spmv<false, DIRECT>(P, lay64, x, S, dyn, pp, er)) return;
     __syncthreads();
     double bbp = 0.0;
     MF_PAIRS(4, vlo, vhi, {
@@ -989,7 +1119,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
         if (pending || (P.replace_every > 0 && it > 0 && it % P.replace_every == 0)) {
             if (!wait_deps(P, S, lay64, ep)) return;
             EpiResidual e2{b, r, 0.0, vpol};
-            if (!cta_spmv<false>(P, lay64, x, S, dyn, pp, e2)) return;
+            if (!cta_spmv<false, DIRECT>(P, lay64, x, S, dyn, pp, e2)) return;
             double v1[1] = {e2.rr}, o1[1];
             if (!grid_sum<1>(P, S, v1, o1, phase)) return;
             const double rr_rec = rr;
@@ -1044,7 +1174,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
         EpiQ eq{d, q, 0.0, vpol};
         bool ok;
         if (MIXED && lay != lay64) ok = cta_spmv<true>(P, lay, P.lay[lay].x32 ? (const void *)d32 : d, S, dyn, pp, eq);
-        else ok = cta_spmv<false>(P, lay64, d, S, dyn, pp, eq);
+        else ok = cta_spmv<false, DIRECT>(P, lay64, d, S, dyn, pp, eq);
         if (!ok) return;
         MF_TRACE(it, 2);
         double v1[1] = {eq.dq}, o1[1];
@@ -2816,6 +2946,8 @@ __global__ void k_residual_norms(int n, const double *b, const double *ax, doubl
 // the single-system kernel on it with the system's gs-CTA slab layout:
 // reductions and halo flags stay inside the group, so groups never wait for
 // each other and many systems are in flight at once.
+// DIRECT: every system's layout is direct.
+template <bool DIRECT>
 __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ Smem S;
@@ -2823,7 +2955,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
     __shared__ int s_rng[4];  // own rows lo, hi; halo ranks lo, hi
     KParams P0;  // only the fields kernel_setup reads
     P0.nlay = 0;
-    P0.stage_stride = B.stage_stride;
+    P0.stage_stride = DIRECT ? 0 : B.stage_stride;
     P0.slab_area = B.slab_area;
     kernel_setup(P0, S, 0);
     const int tid = threadIdx.x;
@@ -2841,6 +2973,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
     uint32_t phase = 0, ep = 0;
     const uint64_t vpol = policy_evict_last();
     const PipeCfg C{B.stage_stride, B.slab_area, B.limit_ns, X.sync, 0};
+    auto spmv = [&](const double *xv, auto &epi) -> bool {
+        if constexpr (DIRECT) {
+            cta_spmv_direct<DIRECT_GB>(D.slabs, D.rbtab, s_rng[0] >> 4, s_rng[1] >> 4, D.gt.rowA, xv, epi);
+            return S.abort == 0;
+        } else {
+            return cta_spmv_src<false, std::remove_reference_t<decltype(epi)>, 8>(L, C, xv, S, dyn, pp, epi);
+        }
+    };
     const bool fixed = B.fixed_iterations > 0;
     const int maxit = fixed ? B.fixed_iterations : B.maxiter;
     while (true) {
@@ -2853,8 +2993,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
         const int sys = B.order[qi];
         if (tid == 0) D = B.sys[sys];  // the group_sum above ended with a barrier
         __syncthreads();
-        const uint8_t *hsrc = D.head + (size_t)rank * STAGES * ISSUE_REC;
-        for (int i = tid; i < STAGES * ISSUE_REC; i += NTHREADS) (&S.head[0][0][0])[i] = hsrc[i];
+        if constexpr (!DIRECT) {
+            const uint8_t *hsrc = D.head + (size_t)rank * STAGES * ISSUE_REC;
+            for (int i = tid; i < STAGES * ISSUE_REC; i += NTHREADS) (&S.head[0][0][0])[i] = hsrc[i];
+        }
         if (tid == 0) {
             L.slabs = D.slabs;
             L.head = &S.head[0][0][0];
@@ -2874,7 +3016,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
         __syncthreads();
         // r = b - A x0, d = r (x0 is written before the launch: no halo wait)
         EpiResidual er{D.b, D.r, 0.0, vpol};
-        if (!cta_spmv_src<false, EpiResidual, 8>(L, C, D.x, S, dyn, pp, er)) return;
+        if (!spmv(D.x, er)) return;
         double bbp = 0.0;
         MF_PAIRS(4, s_rng[0], s_rng[1], {
             double2 rv[_vb], bv[_vb];
@@ -2900,7 +3042,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
         while (it < maxit && (fixed || rel > B.tol)) {
             if (!wait_deps_x(X, S, s_rng[2], s_rng[3], ep)) return;
             EpiQ eq{D.d, D.q, 0.0, vpol};
-            if (!cta_spmv_src<false, EpiQ, 8>(L, C, D.d, S, dyn, pp, eq)) return;
+            if (!spmv(D.d, eq)) return;
             double v1[1] = {eq.dq}, o1[1];
             if (!group_sum<1>(X, S, v1, o1, phase)) return;
             const double dq = o1[0];
@@ -2990,7 +3132,8 @@ int kernel_config(mf_tiles *t, int *G_out) {
     const void *kerns[] = {(const void *)k_cg<false>, (const void *)k_cg<true>, (const void *)k_bicgstab<false>,
                            (const void *)k_bicgstab<true>,
                            (const void *)k_spmv<false>, (const void *)k_spmv<true>, (const void *)k_cgcg,
-                           (const void *)k_batch_cg, (const void *)k_cgcg_tm, (const void *)k_pcg,
+                           (const void *)k_batch_cg<false>, (const void *)k_batch_cg<true>,
+                           (const void *)k_cg<false, true>, (const void *)k_cgcg_tm, (const void *)k_pcg,
                            (const void *)k_cg_tm, (const void *)k_pcg_tm};
     int occ_min = 1 << 30;
     for (const void *k : kerns) {
@@ -3012,6 +3155,7 @@ int kernel_config(mf_tiles *t, int *G_out) {
 
 static void fill_layout_args(LayoutArgs &a, const Layout &L) {
     a.kind = L.kind;
+    a.rbtab = L.direct ? L.rbtab.p : nullptr;
     a.x32 = L.x32 ? 1 : 0;
     a.slabs = L.slabs.p;
     a.head = L.head.p;
@@ -3078,15 +3222,27 @@ int launch_spmv(mf_tiles *t, int level, const void *x, double *y, int reps, cuda
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (!mixed && t->L64.direct) {
+        // one wave of CTAs
+        cfg.gridDim = dim3(std::min((t->tilem + DIRECT_THREADS / 16 - 1) / (DIRECT_THREADS / 16), t->nsm * DIRECT_CTAS));
+        cfg.blockDim = dim3(DIRECT_THREADS);
+        cfg.dynamicSmemBytes = 0;
+        for (int i = 0; i < reps; ++i)
+            MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmv_direct, (const uint8_t *)t->L64.slabs.p,
+                                           (const RbEntry *)t->L64.rbtab.p, t->tilem, t->rowA, (const double *)x, y));
+        return MF_OK;
+    }
     if (mixed) MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmv<true>, P, x, y, lay, reps));
     else MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_spmv<false>, P, x, y, lay, reps));
     return MF_OK;
 }
 
 int launch_solver(mf_tiles *t, int kind, KParams &P, cudaStream_t s) {
-    const int dyn = dyn_smem(t->L64.slab_max);
+    int dyn = dyn_smem(t->L64.slab_max);
+    if (kind == 0 && P.nlay == 1 && P.lay[0].rbtab) dyn = P.stage_stride = 0;  // no ring: all of L1 for x
     void *args[] = {&P};
-    const void *k = kind == 0   ? (P.nlay > 1 ? (const void *)k_cg<true> : (const void *)k_cg<false>)
+    const void *k = kind == 0   ? (P.nlay > 1 ? (const void *)k_cg<true>
+                                   : P.lay[0].rbtab ? (const void *)k_cg<false, true> : (const void *)k_cg<false>)
                     : kind == 2 ? (const void *)k_cgcg
                     : kind == 3 ? (const void *)k_cgcg_tm
                     : kind == 4 ? (const void *)k_pcg
@@ -3097,20 +3253,21 @@ int launch_solver(mf_tiles *t, int kind, KParams &P, cudaStream_t s) {
     return MF_OK;
 }
 
-int launch_batch(const BatchParams &B, int grid, cudaStream_t s) {
+int launch_batch(const BatchParams &B, int grid, bool direct, cudaStream_t s) {
     // cooperative: the CTAs of a group wait on each other, so all must be
     // resident at once (the launch fails instead of deadlocking)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = STAGES * (size_t)B.stage_stride;
+    cfg.dynamicSmemBytes = direct ? 0 : STAGES * (size_t)B.stage_stride;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch_cg, B));
+    if (direct) MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch_cg<true>, B));
+    else MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch_cg<false>, B));
     return MF_OK;
 }
 

@@ -31,6 +31,7 @@ struct LayoutArgs {
     const uint8_t *slabs;
     const uint8_t *head;
     const int *cta_slab, *cta_rb, *cta_dep;
+    const RbEntry *rbtab;  // direct layouts, else nullptr
     int kind;  // LAYOUT_*
     int x32;   // x staged in FP32: the SpMV input is an FP32 vector
 };
@@ -80,6 +81,7 @@ struct SysDesc {
     const uint8_t *head;   // STAGES issue records per CTA of the group
     const int *cta_slab, *cta_rb, *cta_dep;  // per-rank slab / row-block ranges, halo ranks
     int ns, kind;
+    const RbEntry *rbtab;  // direct layouts, else nullptr
     GTiles gt;             // tile arrays (oversize row blocks)
     double *b, *x, *r, *d, *q;  // 16*tilem entries each
     int n16, pad;
@@ -101,7 +103,8 @@ struct BatchParams {
     double *gpartial;     // per group: partial_words(gs), zero before the launch
     BatchResult *res;
 };
-int launch_batch(const BatchParams &B, int grid, cudaStream_t s);
+// direct: every system has a direct layout (SysDesc::rbtab).
+int launch_batch(const BatchParams &B, int grid, bool direct, cudaStream_t s);
 
 int kernel_config(mf_tiles *t, int *G_out);
 void base_params(mf_tiles *t, KParams &P);

@@ -186,6 +186,13 @@ struct RbDir {
                    // the row block's own column segment (0: not staged)
 };
 
+// A row block of a direct layout: an FP64 layout whose slabs are all in gather
+// mode. Its blocks are read where they lie, without the copy ring.
+struct RbEntry {
+    uint32_t off16;  // block's offset from the layout's start, in 16 bytes
+    uint32_t W;      // planes
+};
+
 // Layout kinds: every tile FP64 / every tile below FP64 / both.
 enum { LAYOUT_FP64 = 0, LAYOUT_LOW = 1, LAYOUT_ANY = 2 };
 
@@ -235,6 +242,7 @@ struct Layout {
     DevArray<int> cta_slab;      // G+1: slab range of each CTA
     DevArray<int> cta_rb;        // G+1: row-block range of each CTA
     DevArray<int> cta_dep;       // 2G: CTA range whose vector entries a CTA reads
+    DevArray<RbEntry> rbtab;     // direct layouts (every row block in gather mode): one per row block
     DevArray<uint8_t> prec_dev;  // per tile precision
     DevArray<float> scale_dev;   // per tile scale (FP16 / FP8)
     std::vector<uint8_t> prec;   // host copy of the precisions
@@ -248,6 +256,7 @@ struct Layout {
     double alg_bytes = 0;        // algorithmic bytes of one SpMV
     double tile_frac[4] = {0, 0, 0, 0};
     bool built = false;
+    bool direct = false;         // rbtab is filled
 };
 
 }  // namespace mf
@@ -260,6 +269,7 @@ struct mf_tiles {
     int device = 0, nsm = 0;
     int G = 0;  // persistent CTAs
     mf_options opt;
+    bool all_gather = false;  // plan the FP64 layout in gather mode only (batched systems)
     // Tile_create arrays (device); tile_off is tile_nnz == blknnz == csr_offset
     mf::DevArray<int> tile_ptr, tile_col, tile_off, csrptr_off;
     mf::DevArray<double> val;
