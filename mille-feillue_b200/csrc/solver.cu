@@ -441,6 +441,7 @@ struct SpmvSrc {
     int ns, kind, site;
     int resident_ok;      // slabs may stay in the ring between SpMVs (site = layout index)
     int x32;              // x staged in FP32 (the input vector is FP32)
+    int keep;             // 1/256ths of the slabs copied with evict_normal, the others evict_first
     GTiles gt;
 };
 struct PipeCfg {
@@ -496,7 +497,8 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
         // the first slab of a CTA waiting, which every SpMV of a solve pays:
         // 5-point 256^2 1.73 -> 1.47 us, 7-point 75^3 7.1 -> 6.7 us, 128^3
         // standalone 27.4 -> 26.9 us.
-        const uint64_t pm = policy_evict_first(), pv = policy_evict_last();
+        const uint64_t pm = policy_evict_first(), pk = policy_evict_normal(), pv = policy_evict_last();
+        const int nkeep = (ns * L.keep) >> 8;
         const uint32_t segb = L.x32 ? 64u : 128u;  // an x segment: 16 entries
         fence_proxy_async_global();
         for (int i = 0; i < ns; ++i) {
@@ -545,7 +547,7 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
             if (lane == 0) {
                 mbar_arrive_expect_tx(&S.full[k], held ? xbytes : bytes + xbytes);
                 if (!held) {
-                    bulk_g2s(st, L.slabs + (size_t)off16 * 16, bytes, &S.full[k], pm);
+                    bulk_g2s(st, L.slabs + (size_t)off16 * 16, bytes, &S.full[k], i < nkeep ? pk : pm);
                     S.res_tag[k] = keep ? (uint8_t)(L.site + 1) : (uint8_t)0;
                 }
             }
@@ -765,6 +767,7 @@ __device__ bool cta_spmv(const KParams &P, int lay, const void *xv, Smem &S, uin
     L.ns = S.slab1[lay] - S.slab0[lay];
     L.kind = P.lay[lay].kind;
     L.x32 = P.lay[lay].x32;
+    L.keep = P.lay[lay].keep;
     L.site = lay;
     L.resident_ok = 1;
     L.gt = gtiles_of(P);
@@ -3005,6 +3008,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_batch_cg(BatchParams B) {
             L.site = 40;
             L.resident_ok = 1;  // within this system's solve
             L.x32 = 0;          // FP64 layouts
+            L.keep = 0;         // other groups stream through L2
             L.gt = D.gt;
             s_rng[0] = 16 * D.cta_rb[rank];
             s_rng[1] = 16 * D.cta_rb[rank + 1];
@@ -3157,6 +3161,7 @@ static void fill_layout_args(LayoutArgs &a, const Layout &L) {
     a.kind = L.kind;
     a.rbtab = L.direct ? L.rbtab.p : nullptr;
     a.x32 = L.x32 ? 1 : 0;
+    a.keep = 0;
     a.slabs = L.slabs.p;
     a.head = L.head.p;
     a.cta_slab = L.cta_slab.p;

@@ -34,6 +34,7 @@ struct LayoutArgs {
     const RbEntry *rbtab;  // direct layouts, else nullptr
     int kind;  // LAYOUT_*
     int x32;   // x staged in FP32: the SpMV input is an FP32 vector
+    int keep;  // 1/256ths of each CTA's slabs that stay in L2 between SpMVs
 };
 
 struct DevResult {

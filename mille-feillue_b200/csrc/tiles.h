@@ -266,7 +266,7 @@ constexpr int MF_NLEVELS = 3;
 struct mf_tiles {
     int rowA = 0, colA = 0, tilem = 0, tilen = 0, tilenum = 0, csrsize = 0, csrptrlen = 0;
     int cnt_non_new = 0;
-    int device = 0, nsm = 0;
+    int device = 0, nsm = 0, l2_bytes = 0;
     int G = 0;  // persistent CTAs
     mf_options opt;
     bool all_gather = false;  // plan the FP64 layout in gather mode only (batched systems)
