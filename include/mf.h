@@ -123,7 +123,9 @@ typedef struct {
                                 bytes the launched kernel moves per row and
                                 iteration (56 with vectors in global memory;
                                 28 mixed and 32 FP64 CG, 40 Jacobi PCG with
-                                x and r in tensor memory; 88 BiCGSTAB)        */
+                                x and r in tensor memory; 8 CG and Jacobi PCG
+                                of systems small enough for the chip; 88
+                                BiCGSTAB)                                     */
     int fell_back_fp64;      /* 1 if a low-precision level let the true
                                 residual grow and the solve finished on the
                                 FP64 layout                                   */

@@ -554,6 +554,9 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     // x and r stay in tensor memory when every CTA's rows fit it, the ring
     // holds the vector passes' copies, and one CTA runs per SM (each CTA
     // allocates all of the SM's tensor memory)
+    // small systems: the matrix stays in the ring, the vectors in registers
+    if (!mixed && (launch_kind == 0 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1)
+        launch_kind = launch_kind == 4 ? 8 : 7;
     if ((launch_kind == 2 || launch_kind == 4 || (launch_kind == 0 && !mixed)) && opt.reserved[5] != 1 &&
         t->G == t->nsm && !(launch_kind == 0 && t->L64.direct)) {
         int rows_max = 0;
@@ -627,12 +630,14 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
         // likewise), Jacobi PCG 72 (+ 1/a_ii); with x and r in tensor memory:
         // single-reduction CG 28 (p, s, w in; p, s and the FP32 copy of r
         // out; w from the SpMV), FP64 CG 32 (q, d in; q, d out), Jacobi PCG
-        // 40 (q, d and the FP32 1/a_ii twice in; q, d out)
+        // 40 (q, d and the FP32 1/a_ii twice in; q, d out); with the vectors
+        // in registers 8 (d out)
         const double vpr = kind == 1 ? (P.nlay > 1 ? 136.0 : 112.0)
                            : launch_kind == 3 ? 28.0
                            : launch_kind == 5 ? 32.0
                            : launch_kind == 6 ? 40.0
                            : launch_kind == 4 ? 72.0
+                           : launch_kind >= 7 ? 8.0
                                               : 56.0;
         const double vec = vpr * (double)n;
         const double nsp = kind == 1 ? 2.0 : 1.0;

@@ -881,31 +881,37 @@ __device__ void publish_x(const Ctx &X, uint32_t ep) {
 }
 __device__ void publish(const KParams &P, uint32_t ep) { publish_x(ctx_of(P), ep); }
 
-// Wait until the group's CTAs lo..hi (whose rows this CTA reads) have
-// published epoch `ep`.
-__device__ bool wait_deps_x(const Ctx &X, Smem &S, int lo, int hi, uint32_t ep) {
-    if (threadIdx.x < 32) {
-        for (int c = lo + (int)threadIdx.x; c <= hi; c += 32) {
-            const uint32_t *f = X.sync + SYNC_FLAGS + c * FLAG_STRIDE;
-            if (ld_acquire(f) >= ep) continue;
-            const uint64_t t0 = globaltimer();
-            for (uint32_t spin = 1;; ++spin) {
-                if (ld_acquire(f) >= ep) break;
-                if ((spin & 63u) == 0) {
-                    if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
-                        S.abort = 1;
-                        break;
-                    }
-                    if (globaltimer() - t0 > X.limit_ns) {
-                        set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, 20);
-                        S.abort = 1;
-                        break;
-                    }
+// One warp: waits until the group's CTAs lo..hi (whose rows this CTA reads)
+// have published epoch `ep`. False (and S.abort) when a lane's wait ended
+// without its flags.
+__device__ __forceinline__ bool poll_deps(const Ctx &X, Smem &S, int lo, int hi, uint32_t ep) {
+    bool ok = true;
+    for (int c = lo + (int)(threadIdx.x & 31); c <= hi && ok; c += 32) {
+        const uint32_t *f = X.sync + SYNC_FLAGS + c * FLAG_STRIDE;
+        if (ld_acquire(f) >= ep) continue;
+        const uint64_t t0 = globaltimer();
+        for (uint32_t spin = 1;; ++spin) {
+            if (ld_acquire(f) >= ep) break;
+            if ((spin & 63u) == 0) {
+                if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
+                    ok = false;
+                    break;
+                }
+                if (globaltimer() - t0 > X.limit_ns) {
+                    set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, 20);
+                    ok = false;
+                    break;
                 }
             }
         }
-        __syncwarp();
     }
+    if (!ok) S.abort = 1;
+    __syncwarp();
+    return ok;
+}
+// The same for the whole block.
+__device__ bool wait_deps_x(const Ctx &X, Smem &S, int lo, int hi, uint32_t ep) {
+    if (threadIdx.x < 32) poll_deps(X, S, lo, hi, ep);
     __syncthreads();
     return S.abort == 0;
 }
@@ -2560,6 +2566,191 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_pcg_tm(KParams P) {
     if (w == 0) tmem_dealloc512(s_tmem);
 }
 
+// --------------------------------------- CG and Jacobi PCG, all on the chip
+// Small systems (L64.resident: at most 4 slabs of 30 row blocks a CTA, 148 x
+// 1920 rows in all): the slabs stay in the ring for the whole solve, lane r
+// of half-warp j owns row 16 (rb0 + j) + r of each slab, and x, r, d and q of
+// its rows (up to 4) stay in its registers. An iteration moves the halo of d
+// (8 bytes a row out, the x windows in) and two grid sums; such systems are
+// bound by the latency of these, and the vector passes through tensor memory
+// and the ring (k_cg_tm) cost as much again.
+
+// One SpMV with input xv: the producer warp waits for the neighbours' epoch
+// `ep` (0: nothing to wait for) and copies the x windows (`load`: and the
+// slabs); fin(i, row, acc) for this lane's row of each slab, row < 0 where it
+// has none. par: parity of the stages' full barriers. The caller's barriers
+// keep a window in place until every lane has read it.
+template <class F>
+__device__ __forceinline__ void res_spmv(const KParams &P, Smem &S, uint8_t *dyn, const double *xv, uint32_t ep,
+                                         bool load, uint32_t &par, F fin) {
+    const int ns = S.slab1[0] - S.slab0[0];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w == PRODUCER_WARP) {
+        const Ctx X = ctx_of(P);
+        const bool ok = ep == 0u || poll_deps(X, S, P.lay[0].cta_dep[2 * blockIdx.x],
+                                              P.lay[0].cta_dep[2 * blockIdx.x + 1], ep);
+        if (__all_sync(0xffffffffu, ok)) {
+            const uint64_t pm = policy_evict_first(), pv = policy_evict_last();
+            fence_proxy_async_global();
+            fence_proxy_async_smem();
+            for (int i = 0; i < ns; ++i) {
+                const uint32_t *rec = reinterpret_cast<const uint32_t *>(&S.head[0][i][0]);
+                const int nruns = (int)rec[3];
+                uint8_t *st = stage_ptr(dyn, i, P.stage_stride);
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&S.full[i], rec[2] + (load ? rec[1] : 0u));
+                    if (load) bulk_g2s(st, P.lay[0].slabs + (size_t)rec[0] * 16, rec[1], &S.full[i], pm);
+                }
+                __syncwarp();
+                if (lane < nruns) {
+                    const XRun run = reinterpret_cast<const XRun *>(rec + 4)[lane];
+                    bulk_g2s(st + P.slab_area + (size_t)run.slot0 * 128u, xv + (size_t)run.seg0 * 16,
+                             (uint32_t)run.nseg * 128u, &S.full[i], pv);
+                }
+            }
+        }
+    } else {
+        const int j = 2 * w + (lane >> 4), r = lane & 15;
+#pragma unroll
+        for (int i = 0; i < STAGES; ++i) {
+            if (i < ns) {
+                if (!wait_bar(&S.full[i], par, P.limit_ns)) {
+                    set_error(P, (uint32_t)MF_ERR_TIMEOUT, 120);
+                    S.abort = 1;
+                    break;
+                }
+                const uint8_t *st = stage_ptr(dyn, i, P.stage_stride);
+                const SlabHeader &h = *reinterpret_cast<const SlabHeader *>(st);
+                int row = -1;
+                double acc = 0.0;
+                if (j < (int)h.nrb) {
+                    row = (h.rb0 + j) * 16 + r;
+                    acc = slab_row<LAYOUT_FP64, 1>(st, h, j, r, reinterpret_cast<const double *>(st + P.slab_area), xv);
+                    if (row >= P.rowA) row = -1;
+                }
+                fin(i, row, acc);
+            }
+        }
+    }
+    par ^= 1u;
+}
+
+// The recurrences of k_cg<false> (PCG false) and k_pcg (PCG true).
+template <bool PCG>
+__global__ void __launch_bounds__(NTHREADS, 1) k_cg_res(KParams P) {
+    extern __shared__ __align__(128) uint8_t dyn[];
+    __shared__ Smem S;
+    kernel_setup(P, S, 1);
+    const int g = blockIdx.x, tid = threadIdx.x;
+    uint32_t phase = 0, par = 0;
+    if (P.inject_wait) {
+        // test hook (as in k_cg): an epoch no CTA publishes
+        if (!wait_deps(P, S, 0, 0xffffffffu)) return;
+    }
+    double x[STAGES], r[STAGES], d[STAGES], q[STAGES], m[PCG ? STAGES : 1];
+    int row[STAGES];
+#pragma unroll
+    for (int i = 0; i < STAGES; ++i) {
+        x[i] = r[i] = d[i] = q[i] = 0.0;
+        row[i] = -1;
+    }
+#define MF_ROWS                          \
+    _Pragma("unroll") for (int i = 0; i < STAGES; ++i) if (row[i] >= 0)
+    // r = b - A x0, d = r (z)
+    double rrp = 0.0, rzp = 0.0, bbp = 0.0;
+    res_spmv(P, S, dyn, P.x, 0u, true, par, [&](int i, int rw, double acc) {
+        row[i] = rw;
+        if (rw < 0) return;
+        x[i] = P.x[rw];
+        const double bv = P.b[rw];
+        r[i] = bv - acc;
+        rrp += r[i] * r[i];
+        bbp += bv * bv;
+        if constexpr (PCG) {
+            m[i] = P.s[rw];
+            d[i] = m[i] * r[i];
+            rzp += r[i] * d[i];
+        } else {
+            d[i] = r[i];
+        }
+        P.d[rw] = d[i];
+    });
+    double v3[3] = {rrp, bbp, rzp}, o3[3];
+    if (!grid_sum<3>(P, S, v3, o3, phase)) return;
+    double rr = o3[0], rz = PCG ? o3[2] : o3[0];  // rz: r.z, r.r without a preconditioner
+    const double bb = o3[1];
+    const double bnorm = sqrt(bb);
+    const double tol = P.tol;
+    uint32_t ep = 1;
+    publish(P, ep);
+    int it = 0, status = MF_OK;
+    double rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
+    const bool fixed = P.fixed_iterations > 0;
+    const int maxit = fixed ? P.fixed_iterations : P.maxiter;
+    while (it < maxit && (fixed || rel > tol)) {
+        MF_TRACE(it, 0);
+        MF_TRACE(it, 1);
+        double dqp = 0.0;
+        res_spmv(P, S, dyn, P.d, ep, false, par, [&](int i, int rw, double acc) {
+            q[i] = acc;
+            if (rw >= 0) dqp += d[i] * acc;
+        });
+        MF_TRACE(it, 2);
+        double v1[1] = {dqp}, o1[1];
+        if (!grid_sum<1>(P, S, v1, o1, phase)) return;
+        MF_TRACE(it, 3);
+        const double dq = o1[0];
+        if (!(dq != 0.0) || !isfinite(dq)) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+        const double alpha = rz / dq;
+        rrp = rzp = 0.0;
+        MF_ROWS {
+            r[i] -= alpha * q[i];
+            rrp += r[i] * r[i];
+            if constexpr (PCG) rzp += r[i] * (m[i] * r[i]);
+        }
+        MF_TRACE(it, 4);
+        double w2[PCG ? 2 : 1] = {rrp}, u2[PCG ? 2 : 1];
+        if constexpr (PCG) w2[1] = rzp;
+        if (!grid_sum<PCG ? 2 : 1>(P, S, w2, u2, phase)) return;
+        MF_TRACE(it, 5);
+        rr = u2[0];
+        const double rzn = PCG ? u2[PCG ? 1 : 0] : rr;
+        const double beta = rzn / rz;
+        rz = rzn;
+        ++it;
+        rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
+        MF_ROWS {
+            x[i] += alpha * d[i];
+            d[i] = (PCG ? m[PCG ? i : 0] * r[i] : r[i]) + beta * d[i];
+            P.d[row[i]] = d[i];
+        }
+        ++ep;
+        publish(P, ep);
+        MF_TRACE(it - 1, 6);
+        if (!isfinite(rr)) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+    }
+    MF_ROWS P.x[row[i]] = x[i];
+#undef MF_ROWS
+    if (g == 0 && tid == 0) {
+        if (status == MF_OK && !fixed && rel > tol) status = MF_ERR_NOT_CONVERGED;
+        P.res->iterations = it;
+        P.res->status = status;
+        P.res->replacements = 0;
+        P.res->level_switches = 0;
+        P.res->rr = rr;
+        P.res->bb = bb;
+        P.res->final_layout = 0;
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = l == 0 ? it : 0;
+        P.res->pad = 0;
+    }
+}
+
 // -------------------------------------------------------------- BiCGSTAB
 struct EpiDot {  // y = A p, dot += z*y
     static constexpr bool kUsesX = false;
@@ -3138,7 +3329,8 @@ int kernel_config(mf_tiles *t, int *G_out) {
                            (const void *)k_spmv<false>, (const void *)k_spmv<true>, (const void *)k_cgcg,
                            (const void *)k_batch_cg<false>, (const void *)k_batch_cg<true>,
                            (const void *)k_cg<false, true>, (const void *)k_cgcg_tm, (const void *)k_pcg,
-                           (const void *)k_cg_tm, (const void *)k_pcg_tm};
+                           (const void *)k_cg_tm, (const void *)k_pcg_tm, (const void *)k_cg_res<false>,
+                           (const void *)k_cg_res<true>};
     int occ_min = 1 << 30;
     for (const void *k : kerns) {
         MF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -3253,6 +3445,8 @@ int launch_solver(mf_tiles *t, int kind, KParams &P, cudaStream_t s) {
                     : kind == 4 ? (const void *)k_pcg
                     : kind == 5 ? (const void *)k_cg_tm
                     : kind == 6 ? (const void *)k_pcg_tm
+                    : kind == 7 ? (const void *)k_cg_res<false>
+                    : kind == 8 ? (const void *)k_cg_res<true>
                                 : (P.nlay > 1 ? (const void *)k_bicgstab<true> : (const void *)k_bicgstab<false>);
     MF_CUDA_TRY(cudaLaunchCooperativeKernel(k, dim3(t->G), dim3(NTHREADS), args, dyn, s));
     return MF_OK;

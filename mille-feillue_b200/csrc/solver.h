@@ -12,6 +12,7 @@ namespace mf {
 constexpr int NWARPS = 15;                 // consumer warps per CTA (2 row blocks each)
 constexpr int PRODUCER_WARP = NWARPS;      // one more warp issues the bulk copies
 constexpr int NTHREADS = (NWARPS + 1) * 32;
+static_assert(RB_PER_SLAB_X64 <= 2 * NWARPS, "resident layouts: one row block a half-warp and slab");
 constexpr int KMAX_LAYOUTS = 1 + MF_NLEVELS;
 constexpr int FLAG_STRIDE = 8;             // one 32-byte sector per CTA flag
 enum { SYNC_ERROR = 32, SYNC_SITE = 33, SYNC_FLAGS = 64 };
@@ -114,7 +115,9 @@ int launch_spmv(mf_tiles *t, int level, const void *x, double *y, int reps, cuda
 // dst[0..n) = (float)src[0..n), dst[n..npad) = 0.
 int launch_to_f32(int n, const double *src, float *dst, size_t npad, cudaStream_t s);
 // kind 0 CG, 1 BiCGSTAB, 2 single-reduction CG, 3 the same with x and r in
-// TMEM (every CTA's rows <= TMEM_ROWS_MAX), 4 Jacobi-preconditioned CG.
+// TMEM (every CTA's rows <= TMEM_ROWS_MAX), 4 Jacobi-preconditioned CG, 5 / 6
+// FP64 CG / Jacobi PCG with x and r in TMEM, 7 / 8 the same with the matrix
+// in the ring and the vectors in registers (L64.resident).
 constexpr int TMEM_ROWS_MAX = 128 * 128;
 // The TMEM kernel's vector pass copies 12 bytes per own row into the ring.
 inline bool tm_vectors_fit(int rows_max, int slab_max) {

@@ -257,6 +257,7 @@ struct Layout {
     double tile_frac[4] = {0, 0, 0, 0};
     bool built = false;
     bool direct = false;         // rbtab is filled
+    bool resident = false;       // FP64: every CTA's slabs fit the ring at once, one row block a half-warp each
 };
 
 }  // namespace mf
