@@ -94,9 +94,9 @@ typedef struct {
                                 reserved[4] = CTAs per system group of
                                 mf_batch_create (0 = chosen from the
                                 systems' sizes); reserved[5] = 1:
-                                the CG kernels (FP64 and single-reduction
-                                mixed) keep x and r in global memory
-                                instead of tensor memory;
+                                the solver kernels keep their vectors in
+                                global memory instead of tensor memory or
+                                registers;
                                 reserved[6] = N > 0: reference iteration
                                 count for the learned selector's fallback   */
 } mf_options;
@@ -123,9 +123,9 @@ typedef struct {
                                 bytes the launched kernel moves per row and
                                 iteration (56 with vectors in global memory;
                                 28 mixed and 32 FP64 CG, 40 Jacobi PCG with
-                                x and r in tensor memory; 8 CG and Jacobi PCG
-                                of systems small enough for the chip; 88
-                                BiCGSTAB)                                     */
+                                x and r in tensor memory; 112 FP64, 136 mixed
+                                BiCGSTAB; 8 CG and Jacobi PCG, 16 BiCGSTAB of
+                                systems small enough for the chip)            */
     int fell_back_fp64;      /* 1 if a low-precision level let the true
                                 residual grow and the solve finished on the
                                 FP64 layout                                   */

@@ -555,8 +555,8 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     // holds the vector passes' copies, and one CTA runs per SM (each CTA
     // allocates all of the SM's tensor memory)
     // small systems: the matrix stays in the ring, the vectors in registers
-    if (!mixed && (launch_kind == 0 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1)
-        launch_kind = launch_kind == 4 ? 8 : 7;
+    if (!mixed && (launch_kind <= 1 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1)
+        launch_kind = launch_kind == 4 ? 8 : launch_kind == 1 ? 9 : 7;
     if ((launch_kind == 2 || launch_kind == 4 || (launch_kind == 0 && !mixed)) && opt.reserved[5] != 1 &&
         t->G == t->nsm && !(launch_kind == 0 && t->L64.direct)) {
         int rows_max = 0;
@@ -631,8 +631,9 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
         // single-reduction CG 28 (p, s, w in; p, s and the FP32 copy of r
         // out; w from the SpMV), FP64 CG 32 (q, d in; q, d out), Jacobi PCG
         // 40 (q, d and the FP32 1/a_ii twice in; q, d out); with the vectors
-        // in registers 8 (d out)
-        const double vpr = kind == 1 ? (P.nlay > 1 ? 136.0 : 112.0)
+        // in registers 8 (d out), BiCGSTAB 16 (p and s out)
+        const double vpr = launch_kind == 9 ? 16.0
+                           : kind == 1 ? (P.nlay > 1 ? 136.0 : 112.0)
                            : launch_kind == 3 ? 28.0
                            : launch_kind == 5 ? 32.0
                            : launch_kind == 6 ? 40.0

@@ -2765,6 +2765,137 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg_res(KParams P) {
     }
 }
 
+// The two-reduction recurrence of k_bicgstab<false> in the same form: x, r
+// (then s), p, v, t and r^ of a lane's rows in registers, p and s to global
+// memory for the neighbours' windows.
+__global__ void __launch_bounds__(NTHREADS, 1) k_bicgstab_res(KParams P) {
+    extern __shared__ __align__(128) uint8_t dyn[];
+    __shared__ Smem S;
+    kernel_setup(P, S, 1);
+    const int g = blockIdx.x, tid = threadIdx.x;
+    uint32_t phase = 0, par = 0;
+    double x[STAGES], r[STAGES], p[STAGES], v[STAGES], t[STAGES], rh[STAGES];
+    int row[STAGES];
+#pragma unroll
+    for (int i = 0; i < STAGES; ++i) {
+        x[i] = r[i] = p[i] = v[i] = t[i] = rh[i] = 0.0;
+        row[i] = -1;
+    }
+#define MF_ROWS                          \
+    _Pragma("unroll") for (int i = 0; i < STAGES; ++i) if (row[i] >= 0)
+    // r = b - A x0, r^ = p = r
+    double rrp = 0.0, bbp = 0.0;
+    res_spmv(P, S, dyn, P.x, 0u, true, par, [&](int i, int rw, double acc) {
+        row[i] = rw;
+        if (rw < 0) return;
+        x[i] = P.x[rw];
+        const double bv = P.b[rw];
+        r[i] = rh[i] = p[i] = bv - acc;
+        P.d[rw] = p[i];
+        rrp += r[i] * r[i];
+        bbp += bv * bv;
+    });
+    double v2[2] = {rrp, bbp}, o2[2];
+    if (!grid_sum<2>(P, S, v2, o2, phase)) return;
+    double rr = o2[0], rho = o2[0];
+    const double bb = o2[1];
+    const double bnorm = sqrt(bb);
+    const double tol = P.tol;
+    uint32_t ep = 1;
+    publish(P, ep);
+    int it = 0, status = MF_OK;
+    double rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
+    const bool fixed = P.fixed_iterations > 0;
+    const int maxit = fixed ? P.fixed_iterations : P.maxiter;
+    rrp = 0.0;
+    bool carry = false;  // rrp holds the r.r of an update not yet reduced
+    while (carry || (it < maxit && (fixed || rel > tol))) {
+        double hv = 0.0;
+        res_spmv(P, S, dyn, P.d, ep, false, par, [&](int i, int rw, double acc) {
+            v[i] = acc;
+            if (rw >= 0) hv += rh[i] * acc;
+        });
+        double a1[2] = {hv, rrp}, b1[2];
+        if (!grid_sum<2>(P, S, a1, b1, phase)) return;
+        if (carry) {
+            carry = false;
+            rr = b1[1];
+            rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
+            if (!isfinite(rr)) {
+                status = MF_ERR_BREAKDOWN;
+                break;
+            }
+            if (it >= maxit || (!fixed && rel <= tol)) break;
+        }
+        if (!(b1[0] != 0.0) || !isfinite(b1[0])) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+        const double alpha = rho / b1[0];
+        MF_ROWS {
+            r[i] -= alpha * v[i];  // s
+            P.s[row[i]] = r[i];
+        }
+        ++ep;
+        publish(P, ep);
+        double ts = 0.0, tt = 0.0, hs = 0.0, ht = 0.0;
+        res_spmv(P, S, dyn, P.s, ep, false, par, [&](int i, int rw, double acc) {
+            t[i] = acc;
+            if (rw < 0) return;
+            ts += acc * r[i];
+            tt += acc * acc;
+            hs += rh[i] * r[i];
+            ht += rh[i] * acc;
+        });
+        double a2[4] = {ts, tt, hs, ht}, b2[4];
+        if (!grid_sum<4>(P, S, a2, b2, phase)) return;
+        if (!(b2[1] != 0.0) || !isfinite(b2[1])) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+        const double omega = b2[0] / b2[1];
+        const double rho1 = b2[2] - omega * b2[3];
+        const double beta = omega != 0.0 ? (rho1 * alpha) / (rho * omega) : 0.0;
+        rrp = 0.0;
+        MF_ROWS {
+            x[i] = x[i] + alpha * p[i] + omega * r[i];
+            r[i] -= omega * t[i];
+            p[i] = r[i] + beta * (p[i] - omega * v[i]);
+            P.d[row[i]] = p[i];
+            rrp += r[i] * r[i];
+        }
+        rho = rho1;
+        ++it;
+        carry = true;
+        ++ep;
+        publish(P, ep);
+        if (omega == 0.0) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+    }
+    if (carry) {  // a breakdown left the last update's r.r unreduced
+        double a1[1] = {rrp}, b1[1];
+        if (!grid_sum<1>(P, S, a1, b1, phase)) return;
+        rr = b1[0];
+        rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
+    }
+    MF_ROWS P.x[row[i]] = x[i];
+#undef MF_ROWS
+    if (g == 0 && tid == 0) {
+        if (status == MF_OK && !fixed && rel > tol) status = MF_ERR_NOT_CONVERGED;
+        P.res->iterations = it;
+        P.res->status = status;
+        P.res->replacements = 0;
+        P.res->level_switches = 0;
+        P.res->rr = rr;
+        P.res->bb = bb;
+        P.res->final_layout = 0;
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = l == 0 ? it : 0;
+        P.res->pad = 0;
+    }
+}
+
 // -------------------------------------------------------------- BiCGSTAB
 struct EpiDot {  // y = A p, dot += z*y
     static constexpr bool kUsesX = false;
@@ -3344,7 +3475,7 @@ int kernel_config(mf_tiles *t, int *G_out) {
                            (const void *)k_batch_cg<false>, (const void *)k_batch_cg<true>,
                            (const void *)k_cg<false, true>, (const void *)k_cgcg_tm, (const void *)k_pcg,
                            (const void *)k_cg_tm, (const void *)k_pcg_tm, (const void *)k_cg_res<false>,
-                           (const void *)k_cg_res<true>};
+                           (const void *)k_cg_res<true>, (const void *)k_bicgstab_res};
     int occ_min = 1 << 30;
     for (const void *k : kerns) {
         MF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -3461,6 +3592,7 @@ int launch_solver(mf_tiles *t, int kind, KParams &P, cudaStream_t s) {
                     : kind == 6 ? (const void *)k_pcg_tm
                     : kind == 7 ? (const void *)k_cg_res<false>
                     : kind == 8 ? (const void *)k_cg_res<true>
+                    : kind == 9 ? (const void *)k_bicgstab_res
                                 : (P.nlay > 1 ? (const void *)k_bicgstab<true> : (const void *)k_bicgstab<false>);
     MF_CUDA_TRY(cudaLaunchCooperativeKernel(k, dim3(t->G), dim3(NTHREADS), args, dyn, s));
     return MF_OK;

@@ -116,8 +116,9 @@ int launch_spmv(mf_tiles *t, int level, const void *x, double *y, int reps, cuda
 int launch_to_f32(int n, const double *src, float *dst, size_t npad, cudaStream_t s);
 // kind 0 CG, 1 BiCGSTAB, 2 single-reduction CG, 3 the same with x and r in
 // TMEM (every CTA's rows <= TMEM_ROWS_MAX), 4 Jacobi-preconditioned CG, 5 / 6
-// FP64 CG / Jacobi PCG with x and r in TMEM, 7 / 8 the same with the matrix
-// in the ring and the vectors in registers (L64.resident).
+// FP64 CG / Jacobi PCG with x and r in TMEM, 7 / 8 / 9 FP64 CG / Jacobi PCG /
+// BiCGSTAB with the matrix in the ring and the vectors in registers
+// (L64.resident).
 constexpr int TMEM_ROWS_MAX = 128 * 128;
 // The TMEM kernel's vector pass copies 12 bytes per own row into the ring.
 inline bool tm_vectors_fit(int rows_max, int slab_max) {

@@ -39,3 +39,23 @@ def test_resident_matches_global_vectors(mf, kind, size, solver):
     x, r = f(b, x0=x0, tol=1e-10, maxiter=20000, opts=o5)
     assert r["iterations"] == 5
     assert np.linalg.norm(x - xg) <= 1e-12 * np.linalg.norm(xg)
+
+
+@pytest.mark.parametrize("N", [1, 2, 7, 20, 33, 41, 42, 52, 60, 64])
+def test_resident_bicgstab_matches_global_vectors(mf, N):
+    A = mf.Matrix.convdiff3d(N)
+    b = np.random.default_rng(N).standard_normal(A.n)
+    t = mf.Tiles(A)
+    o = mf.options()
+    o.reserved[5] = 1
+    xg, rg = t.solve_bicgstab(b, tol=1e-10, maxiter=2000, opts=o)
+    x, r = t.solve_bicgstab(b, tol=1e-10, maxiter=2000)
+    assert rg["status"] == 0 and r["status"] == 0
+    assert r["rel_residual_true"] <= 1.5e-10
+    assert abs(r["iterations"] - rg["iterations"]) <= max(2, 0.02 * rg["iterations"])
+    if N > 2:  # (smaller systems are solved exactly before five steps)
+        o.fixed_iterations = 5
+        xg, _ = t.solve_bicgstab(b, tol=1e-10, maxiter=2000, opts=o)
+        x, r = t.solve_bicgstab(b, tol=1e-10, maxiter=2000, opts=mf.options(fixed_iterations=5))
+        assert r["iterations"] == 5
+        assert np.linalg.norm(x - xg) <= 1e-12 * np.linalg.norm(xg)
