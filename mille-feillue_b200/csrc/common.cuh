@@ -83,9 +83,6 @@ MF_DEV uint32_t ld_relaxed(const uint32_t *p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-MF_DEV void st_release(uint32_t *p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 MF_DEV void st_relaxed(uint32_t *p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -113,9 +110,6 @@ MF_DEV uint64_t ld_packet_relaxed(const double *p, double &v) {
         : "memory");
     v = __longlong_as_double(lo);
     return tag;
-}
-MF_DEV void red_release_add(uint32_t *p, uint32_t v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // FP64 vector loads / stores with an L2 eviction-priority policy.

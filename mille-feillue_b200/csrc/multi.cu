@@ -361,8 +361,8 @@ __global__ void k_mr_unpack(int n, int k, const double *panel, double *cm) {
 // 16-byte FP32 or two 16-byte FP64 accesses per panel row), so every panel
 // access is a full 64- or 128-byte line per row and the column partials
 // reduce across the lanes with equal lane & 3. Grid sums: per-CTA partials
-// in a fixed order, a release/acquire arrival counter, every CTA summing the
-// same partials in the same order (all CTAs hold identical scalars, so every
+// as tagged packets, every CTA summing the same partials in the same fixed
+// order (all CTAs hold identical scalars, so every
 // decision is uniform). Every wait is bounded (MF_ERR_TIMEOUT).
 constexpr int MRF_THREADS = 512;
 constexpr int MRF_WARPS = MRF_THREADS / 32;
@@ -394,9 +394,11 @@ struct MrfPlan {
     int staged, nruns, own_slot, nseg;  // own_slot: window row of the block's first row
     MrfRun run[MRF_WIN_RUNS];
 };
+static_assert(MRF_ROWS * 320 <= MRF_WSTAGE_BYTES && MRF_ROWS * 160 <= MRF_STAGE_BYTES, "the x, p pass's chunks");
 static_assert(MRF_THREADS == 512, "the grid sum stages 32 chunks of 16 columns");
 constexpr int MRF_FLAG_STRIDE = 8;  // one 32-byte sector per CTA flag
-enum { MRF_ARRIVE = 0, MRF_ERROR = 32, MRF_SITE = 33, MRF_FLAGS = 64 };
+constexpr int MRF_PACKETS = 2 * KW;     // doubles of a CTA's 16 packets
+enum { MRF_ERROR = 32, MRF_SITE = 33, MRF_FLAGS = 64 };
 
 struct MrfOut {
     double rr[KW], bb[KW];
@@ -419,7 +421,7 @@ struct MrfParams {
     double *X, *R;
     float *P, *Q;
     uint32_t *sync;
-    double *partial;  // [2][G][16]
+    double *partial;  // [2][G][MRF_PACKETS], zero at launch
     const int *dep;   // [G][2]: first and last CTA whose rows this CTA's columns reach
     double tol;
     int maxiter, replace_every;
@@ -451,7 +453,10 @@ __device__ __forceinline__ void mrf_error(uint32_t *sync, uint32_t code, uint32_
 }
 
 // Grid-wide sum of 16 column partials; v[m] is this thread's partial of
-// column 4 (lane & 3) + m. Result in S.bres (every CTA the same bits).
+// column 4 (lane & 3) + m. Result in S.bres (every CTA the same bits). Each
+// CTA's 16 sums go out as packets of {value, phase tag} (16 bytes, one memory
+// operation) and every CTA polls all of them: one trip through L2 where an
+// arrival counter takes two and a release.
 __device__ bool mrf_gsum(const MrfParams &P, MrfShared &S, double (&v)[4], uint32_t &phase) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 #pragma unroll
@@ -464,44 +469,69 @@ __device__ bool mrf_gsum(const MrfParams &P, MrfShared &S, double (&v)[4], uint3
 #pragma unroll
         for (int m = 0; m < 4; ++m) S.red[w][lane * 4 + m] = v[m];
     __syncthreads();
-    const int G = P.G, slot = phase & 1;
+    const int G = P.G;
+    const uint64_t tag = (uint64_t)phase + 1u;
+    double *slot = P.partial + (size_t)(phase & 1u) * G * MRF_PACKETS;
     if (tid < KW) {
         double a = 0.0;
         for (int q = 0; q < MRF_WARPS; ++q) a += S.red[q][tid];
-        P.partial[((size_t)slot * G + blockIdx.x) * KW + tid] = a;
+        st_packet_relaxed(slot + (size_t)blockIdx.x * MRF_PACKETS + 2 * tid, a, tag);
     }
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        red_release_add(P.sync + MRF_ARRIVE, 1u);
-        const uint32_t target = (phase + 1) * (uint32_t)G;
-        if (ld_acquire(P.sync + MRF_ARRIVE) < target) {
-            const uint64_t t0 = globaltimer();
+    __syncthreads();  // polls before the CTA's own store only delay the others'
+    {
+        const int j = tid & 15, c = tid >> 4;  // 32 chunks of CTAs per column
+        constexpr int PK = 5;  // packets of a thread in flight
+        double a = 0.0;
+        bool ok = true;
+#pragma unroll 1
+        for (int g0 = c; g0 < G && ok; g0 += 32 * PK) {
+            double v[PK];
+            uint32_t todo = 0;
+#pragma unroll
+            for (int u = 0; u < PK; ++u) todo |= (g0 + 32 * u < G ? 1u : 0u) << u;
+            uint64_t t0 = 0;
             for (uint32_t spin = 1;; ++spin) {
-                if (ld_acquire(P.sync + MRF_ARRIVE) >= target) break;
+                uint64_t tg[PK];
+                double w[PK];
+#pragma unroll
+                for (int u = 0; u < PK; ++u) {
+                    tg[u] = 0;
+                    w[u] = 0.0;
+                    if ((todo >> u) & 1u) tg[u] = ld_packet_relaxed(slot + (size_t)(g0 + 32 * u) * MRF_PACKETS + 2 * j, w[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < PK; ++u)
+                    if (tg[u] == tag) {
+                        v[u] = w[u];
+                        todo &= ~(1u << u);
+                    }
+                if (todo == 0u) break;
+                const long long t1 = clock64();
+                while (clock64() - t1 < 150) {  // the polls share L2 with the stores they wait for
+                }
                 if ((spin & 63u) == 0) {
+                    if (t0 == 0) t0 = globaltimer();
                     if (ld_relaxed(P.sync + MRF_ERROR) != 0u) {
-                        S.abort = 1;
+                        ok = false;
                         break;
                     }
                     if (globaltimer() - t0 > P.limit_ns) {
                         mrf_error(P.sync, (uint32_t)MF_ERR_TIMEOUT, 1);
-                        S.abort = 1;
+                        ok = false;
                         break;
                     }
                 }
             }
+            if (ok)
+#pragma unroll
+                for (int u = 0; u < PK; ++u)
+                    if (g0 + 32 * u < G) a += v[u];
         }
-    }
-    __syncthreads();
-    if (S.abort) return false;
-    {
-        const int j = tid & 15, c = tid >> 4;  // 32 chunks of CTAs per column
-        double a = 0.0;
-        for (int g = c; g < G; g += 32) a += __ldcg(&P.partial[((size_t)slot * G + g) * KW + j]);
+        if (!ok) S.abort = 1;
         S.chunk[c][j] = a;
     }
     __syncthreads();
+    if (S.abort) return false;
     if (tid < KW) {
         double a = 0.0;
         for (int c = 0; c < 32; ++c) a += S.chunk[c][tid];
@@ -515,8 +545,8 @@ __device__ bool mrf_gsum(const MrfParams &P, MrfShared &S, double (&v)[4], uint3
 __device__ void mrf_publish(const MrfParams &P, uint32_t ep) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        st_release(P.sync + MRF_FLAGS + blockIdx.x * MRF_FLAG_STRIDE, ep);
+        fence_acq_rel_gpu();
+        st_relaxed(P.sync + MRF_FLAGS + blockIdx.x * MRF_FLAG_STRIDE, ep);
     }
 }
 
@@ -1222,7 +1252,9 @@ __global__ void __launch_bounds__(MRF_THREADS, 1) k_mr_fused(MrfParams P) {
             bool live[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) bt[m] = S.beta[4 * cg + m], live[m] = S.live[4 * cg + m] != 0;
-            constexpr int C2 = MRF_ROWS / 2;  // 320 bytes a row: P, R, X
+            // 320 bytes a row (P, R, X): a window mode stage holds a row for
+            // every quarter-warp, the others' stages half as many
+            constexpr int C2 = MODE == MRF_MODE_WIN ? MRF_ROWS : MRF_ROWS / 2;
             auto issue = [&](int rb, int rn, int k) {
                 uint8_t *st = ring.buf + (size_t)k * ring.sb;
                 mbar_arrive_expect_tx(&S.full[k], (uint32_t)rn * (replaced ? 192 : 320));
@@ -1232,7 +1264,6 @@ __global__ void __launch_bounds__(MRF_THREADS, 1) k_mr_fused(MrfParams P) {
                     bulk_g2s(st + C2 * 192, P.X + (size_t)rb * KW, (uint32_t)rn * 128, &S.full[k], ring.pol);
             };
             auto body = [&](int rb, int rn, const uint8_t *st) {
-                // two threads a row-quarter: the pass's chunk is half as many rows
                 if (rs >= rn) return;
                 const int row = rb + rs;
                 const float4 p = reinterpret_cast<const float4 *>(st)[rs * 4 + cg];
@@ -1572,7 +1603,7 @@ int multi_fp32(int n, const int *rp, const int *ci, const double *val, int k, co
     DevArray<MrfOut> out;
     const size_t sync_words = (size_t)MRF_FLAGS + (size_t)G * MRF_FLAG_STRIDE;
     if (pb.alloc(nel) || px.alloc(nel) || pr.alloc(nel) || pp.alloc(nel) || pq.alloc(nel) ||
-        part.alloc((size_t)2 * G * KW) || dep.alloc((size_t)2 * G) || sync.alloc(sync_words) || out.alloc(1))
+        part.alloc((size_t)2 * G * MRF_PACKETS) || dep.alloc((size_t)2 * G) || sync.alloc(sync_words) || out.alloc(1))
         return MF_ERR_NOMEM;
     if (mode == MRF_MODE_WIN) {
         if (pev.alloc(npad * 8) || pec.alloc(npad * 8) || pel.alloc(npad * 8) || plan.alloc(nblk))
@@ -1583,6 +1614,7 @@ int multi_fp32(int n, const int *rp, const int *ci, const double *val, int k, co
         k_mr_pad<<<pk, 256, 0, s>>>(n, W, rp, ci, val, pec.p, pev.p);
     }
     MF_CUDA_TRY(cudaMemsetAsync(sync.p, 0, sync_words * sizeof(uint32_t), s));
+    MF_CUDA_TRY(cudaMemsetAsync(part.p, 0, part.n * sizeof(double), s));  // the packets' phase tags
     MF_CUDA_TRY(cudaMemsetAsync(pb.p, 0, nel * sizeof(double), s));
     MF_CUDA_TRY(cudaMemsetAsync(px.p, 0, nel * sizeof(double), s));
     MF_CUDA_TRY(cudaMemsetAsync(pr.p, 0, nel * sizeof(double), s));
