@@ -49,6 +49,9 @@ struct __align__(16) Smem {
     uint8_t res_tag[STAGES];  // 1 + layout whose slab (index = stage) the stage holds; 0: none
     int slab0[KMAX_LAYOUTS], slab1[KMAX_LAYOUTS];
     double red[NWARPS + 1][4];
+    // thread 0's tallies of a mixed solve (in shared memory: the fences drop
+    // spilled registers and local arrays from L1)
+    int it_layout[KMAX_LAYOUTS], n_repl, n_switch, fellback;
     double chunk[PACKET_VALUES * MAX_CHUNKS];  // group_sum: sums of 32 CTAs' packets
     uint8_t head[KMAX_LAYOUTS][STAGES][ISSUE_REC];
 };
@@ -787,9 +790,9 @@ struct Ctx {
 // Sums NV partials over the block and then over the group, in fixed orders:
 // every CTA holds the identical sums. Thread k < NV adds the warps' shares of
 // value k and stores {share of this CTA, phase tag} as one 16-byte packet
-// (slot [phase & 1][rank][k]). Then each warp takes chunks of 32 CTAs of one
-// value, polls one packet a lane until it carries the tag, and adds the
-// chunk by a shuffle tree; the chunks are added in ascending order.
+// (slot [phase & 1][rank][k]). Then each warp takes a chunk of CTAs of one
+// value, polls a packet a lane until it carries the tag, and adds the chunk
+// by a shuffle tree; the chunks are added in ascending order.
 // Latency-bound: a packet costs one store and one load through L2, where an
 // arrival counter costs a release, the wait on the counter and a second trip
 // for the partials (148 CTAs, 512 threads, one value: 1.4 us against 2.3).
@@ -825,26 +828,25 @@ __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (
     // polls that start before the CTA's own store is out only delay the
     // others' stores (1.66 us without this barrier, 1.35 with it)
     __syncthreads();
-    const int nch = (X.G + 31) >> 5;  // chunks of a value
-    for (int ch = w; ch < NV * nch; ch += NWARPS + 1) {
-        const int k = ch / nch, c = (ch - k * nch) * 32 + lane;
-        __syncwarp();
+    int nch;  // chunks of a value
+    if constexpr (NV == 4) {
+        // 20 chunks of 32 would give some warps two in turn: four warps a
+        // value, two packets a lane at once (us an iteration: mixed CG 128^3
+        // 29.8 -> 28.9, BiCGSTAB 64^3 15.0 -> 14.2)
+        nch = 4;
+        const int span = (X.G + 3) >> 2, lo = (w & 3) * span, hi = min(X.G, lo + span);
         double a = 0.0;
-        if (c < X.G) {
-            const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * k;
+        for (int c = lo + lane; c < hi; c += 64) {
+            const double *p1 = slot + (size_t)c * PACKET_STRIDE + 2 * (w >> 2), *p2 = p1 + 32 * PACKET_STRIDE;
+            bool need1 = true, need2 = c + 32 < hi;
+            double v1 = 0.0, v2 = 0.0;
             uint64_t t0 = 0;
-            for (uint32_t spin = 1; ld_packet_relaxed(pk, a) != tag; ++spin) {
-                // a pause between polls: the polls of the CTAs that wait share
-                // L2 with the stores they wait for. us an iteration with and
-                // without: 5-point CG 256^2 5.6..6.0, 5.8..7.3; Jacobi PCG 75^3
-                // 14.3..14.9, 14.5..16.4; FP64 CG 128^3 38.0, 38.4; not with
-                // four values (mixed CG 29.9, 29.7), whose warps poll a second
-                // chunk next
-                if constexpr (NV <= 2) {
-                    const long long t1 = clock64();
-                    while (clock64() - t1 < 150) {
-                    }
-                }
+            for (uint32_t spin = 1;; ++spin) {
+                double u1 = 0.0, u2 = 0.0;
+                const uint64_t g1 = need1 ? ld_packet_relaxed(p1, u1) : 0u, g2 = need2 ? ld_packet_relaxed(p2, u2) : 0u;
+                if (g1 == tag) v1 = u1, need1 = false;
+                if (g2 == tag) v2 = u2, need2 = false;
+                if (!need1 && !need2) break;
                 if ((spin & 63u) == 0) {
                     if (t0 == 0) t0 = globaltimer();
                     if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
@@ -858,11 +860,49 @@ __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (
                     }
                 }
             }
+            a += v1 + v2;
         }
         __syncwarp();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) S.chunk[ch] = a;
+        if (lane == 0) S.chunk[w] = a;
+    } else {
+        nch = (X.G + 31) >> 5;
+        for (int ch = w; ch < NV * nch; ch += NWARPS + 1) {
+            const int k = ch / nch, c = (ch - k * nch) * 32 + lane;
+            __syncwarp();
+            double a = 0.0;
+            if (c < X.G) {
+                const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * k;
+                uint64_t t0 = 0;
+                for (uint32_t spin = 1; ld_packet_relaxed(pk, a) != tag; ++spin) {
+                    // a pause between polls: the polls of the CTAs that wait
+                    // share L2 with the stores they wait for. us an iteration
+                    // with and without: 5-point CG 256^2 5.6..6.0, 5.8..7.3;
+                    // Jacobi PCG 75^3 14.3..14.9, 14.5..16.4; FP64 CG 128^3
+                    // 38.0, 38.4; not with four values (mixed CG 29.9, 29.7)
+                    const long long t1 = clock64();
+                    while (clock64() - t1 < 150) {
+                    }
+                    if ((spin & 63u) == 0) {
+                        if (t0 == 0) t0 = globaltimer();
+                        if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
+                            S.abort = 1;
+                            break;
+                        }
+                        if (globaltimer() - t0 > X.limit_ns) {
+                            set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, 10);
+                            S.abort = 1;
+                            break;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0) S.chunk[ch] = a;
+        }
     }
     __syncthreads();
     if (S.abort) return false;
@@ -955,6 +995,8 @@ __device__ void kernel_setup(const KParams &P, Smem &S, int nlay) {
         mbar_fence_init();
         S.abort = 0;
         for (int k = 0; k < STAGES; ++k) S.res_tag[k] = 0;
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) S.it_layout[l] = 0;
+        S.n_repl = S.n_switch = S.fellback = 0;
     }
     for (int l = 0; l < nlay; ++l) {
         const uint8_t *src = P.lay[l].head + (size_t)blockIdx.x * STAGES * ISSUE_REC;
@@ -1133,7 +1175,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
     // With true_check, a recursive residual under tol is confirmed with the
     // FP64 true residual b - A x before the solve stops (mixed layouts).
     bool pending = false;
-    int it_lay[KMAX_LAYOUTS] = {0, 0, 0, 0};
     double rr_best = rr;
     int fellback = 0;
     while (it < maxit && (fixed || rel > tol || pending)) {
@@ -1193,7 +1234,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
         MF_TRACE(it, 0);
         if (!wait_deps(P, S, lay, ep)) return;
         MF_TRACE(it, 1);
-        ++it_lay[lay];
+        if (tid == 0) ++S.it_layout[lay];
         EpiQ eq{d, q, 0.0, vpol};
         bool ok;
         if (MIXED && lay != lay64) ok = cta_spmv<true>(P, lay, P.lay[lay].x32 ? (const void *)d32 : d, S, dyn, pp, eq);
@@ -1278,7 +1319,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
         P.res->rr = rr;
         P.res->bb = bb;
         P.res->final_layout = lay;
-        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = it_lay[l];
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = S.it_layout[l];
         P.res->pad = fellback;
     }
     (void)G;
@@ -1517,7 +1558,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cgcg(KParams P) {
     uint32_t ep = 1;
     publish(P, ep);
     int it = 0, status = MF_OK, repl = 0, switches = 0, fellback = 0;
-    int it_lay[KMAX_LAYOUTS] = {0, 0, 0, 0};
     double gamma_old = 0.0, rel = 1.0, rr_best = 1e300, gam = 0.0;
     bool first = true, pending = false;
     const bool fixed = P.fixed_iterations > 0;
@@ -1576,7 +1616,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cgcg(KParams P) {
         MF_TRACE(it, 0);
         if (!wait_deps(P, S, lay, ep)) return;
         MF_TRACE(it, 1);
-        ++it_lay[lay];
+        if (tid == 0) ++S.it_layout[lay];
         EpiW ew{r, wv32, 0.0, 0.0, vpol};
         bool ok;
         if (lay != lay64) ok = cta_spmv<true>(P, lay, P.lay[lay].x32 ? (const void *)r32 : r, S, dyn, pp, ew);
@@ -1664,7 +1704,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cgcg(KParams P) {
         P.res->rr = bnorm > 0 ? rel * rel * bb : gam;
         P.res->bb = bb;
         P.res->final_layout = lay;
-        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = it_lay[l];
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = S.it_layout[l];
         P.res->pad = fellback;
     }
 }
@@ -1927,8 +1967,7 @@ __device__ __forceinline__ void cgcg_tm_body(const KParams &P, Smem &S, uint8_t 
     const double tol = P.tol;
     uint32_t ep = 1;
     publish(P, ep);
-    int it = 0, status = MF_OK, repl = 0, switches = 0, fellback = 0;
-    int it_lay[KMAX_LAYOUTS] = {0, 0, 0, 0};
+    int it = 0, status = MF_OK;
     double gamma_old = 0.0, rel = 1.0, rr_best = 1e300, gam = 0.0;
     bool first = true, pending = false;
     const bool fixed = P.fixed_iterations > 0;
@@ -1964,7 +2003,7 @@ __device__ __forceinline__ void cgcg_tm_body(const KParams &P, Smem &S, uint8_t 
             if (lane == 0) s_wpart[0][wid] = rsl;
             double a1[1] = {gl}, c1[1];
             if (!grid_sum<1>(P, S, a1, c1, phase)) return;
-            ++repl;
+            if (tid == 0) ++S.n_repl;
             ++ep;
             publish(P, ep);
             const double relt = bnorm > 0 ? sqrt(c1[0]) / bnorm : 0.0;
@@ -1983,11 +2022,11 @@ __device__ __forceinline__ void cgcg_tm_body(const KParams &P, Smem &S, uint8_t 
                 if (c1[0] < rr_best) rr_best = c1[0];
                 if (!(c1[0] <= 1e4 * rr_best)) {
                     lay = lay64;
-                    fellback = 1;
+                    if (tid == 0) S.fellback = 1;
                 }
                 while (lay != lay64 && lay < P.nlay - 1 && relt < P.level_rel[lay]) {
                     ++lay;
-                    ++switches;
+                    if (tid == 0) ++S.n_switch;
                 }
             }
         }
@@ -1995,7 +2034,7 @@ __device__ __forceinline__ void cgcg_tm_body(const KParams &P, Smem &S, uint8_t 
         MF_TRACE(it, 0);
         if (!wait_deps(P, S, lay, ep)) return;
         MF_TRACE(it, 1);
-        ++it_lay[lay];
+        if (tid == 0) ++S.it_layout[lay];
         EpiW32 ew{r32, wv32, 0.0, vpol};
         bool ok;
         if (lay != lay64) ok = cta_spmv<true>(P, lay, P.lay[lay].x32 ? (const void *)r32 : r, S, dyn, pp, ew);
@@ -2079,13 +2118,13 @@ __device__ __forceinline__ void cgcg_tm_body(const KParams &P, Smem &S, uint8_t 
         if (status == MF_OK && !fixed && rel > tol) status = MF_ERR_NOT_CONVERGED;
         P.res->iterations = it;
         P.res->status = status;
-        P.res->replacements = repl;
-        P.res->level_switches = switches;
+        P.res->replacements = S.n_repl;
+        P.res->level_switches = S.n_switch;
         P.res->rr = bnorm > 0 ? rel * rel * bb : gam;
         P.res->bb = bb;
         P.res->final_layout = lay;
-        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = it_lay[l];
-        P.res->pad = fellback;
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = S.it_layout[l];
+        P.res->pad = S.fellback;
     }
 }
 
@@ -2992,7 +3031,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_bicgstab(KParams P) {
     uint32_t ep = 1;
     publish(P, ep);
     int it = 0, status = MF_OK, repl = 0, switches = 0, fellback = 0;
-    int it_lay[KMAX_LAYOUTS] = {0, 0, 0, 0};
     double rel = bnorm > 0 ? sqrt(rr) / bnorm : 0.0;
     double rr_best = rr;
     bool pending = false;
@@ -3139,7 +3177,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_bicgstab(KParams P) {
             }
         }
         if (it >= maxit) break;
-        ++it_lay[lay];
+        if (tid == 0) ++S.it_layout[lay];
         if (!wait_deps(P, S, lay, ep)) return;
         EpiDot ev{rh, v, 0.0, vpol};
         bool ok;
@@ -3254,7 +3292,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_bicgstab(KParams P) {
         P.res->rr = rr;
         P.res->bb = bb;
         P.res->final_layout = lay;
-        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = MIXED ? it_lay[l] : (l == 0 ? it : 0);
+        for (int l = 0; l < KMAX_LAYOUTS; ++l) P.res->it_layout[l] = MIXED ? S.it_layout[l] : (l == 0 ? it : 0);
         P.res->pad = fellback;
     }
 }
