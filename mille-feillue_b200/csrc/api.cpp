@@ -103,7 +103,25 @@ int encode_dev_impl(int n, int ncols, int nnz, const int *rp, const int *ci, con
     cudaStream_t s = 0;
     if ((rc = encode_device(t, n, ncols, nnz, rp, ci, val, s)) != MF_OK) { delete t; return rc; }
     std::vector<uint8_t> prec(t->tilenum, MF_PREC_FP64);
+    // A small FP64 system takes about one full slab a CTA instead of every
+    // SM: its solves are bound by the grid sums, which cost more the more CTAs
+    // poll (us an iteration with 148 CTAs and so: 5-point CG 37^2 5.5 -> 5.0,
+    // 90^2 5.9 -> 5.0; Jacobi PCG 13^3 8.5 -> 5.3; BiCGSTAB 16^3 10.7 -> 7.6;
+    // below 16 CTAs little changes, and the SpMV alone slows down). 28 row
+    // blocks a CTA on average leave every range within the slab's 30. Not for
+    // scattered matrices (about one entry a tile) or rows so long that 28 row
+    // blocks need a second slab: those want every SM, and where the estimate
+    // errs the layout is planned again.
+    const int g_all = t->G, g_few = std::max(16, (t->tilem + 27) / 28);
+    if (G_force == 0 && t->opt.precision_mode == MF_MODE_FP64 && 4 * g_few <= 3 * g_all &&
+        t->csrsize >= 2ll * t->tilenum && 12.0 * 28.0 * t->csrsize <= (double)SLAB_MAX_DEFAULT * t->tilem)
+        t->G = g_few;
     if ((rc = build_layout(t, t->L64, prec, s)) != MF_OK) { delete t; return rc; }
+    if (t->G < g_all && !(t->L64.resident && t->L64.slabs_max <= 1)) {
+        t->G = g_all;
+        t->h_cta_rb.clear();
+        if ((rc = build_layout(t, t->L64, prec, s)) != MF_OK) { delete t; return rc; }
+    }
     if (t->opt.precision_mode != MF_MODE_FP64) {
         if ((rc = build_mixed_levels(t, s)) != MF_OK) { delete t; return rc; }
     }
@@ -560,14 +578,14 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
         if (rj) return rj;
     }
     int launch_kind = kind == 2 ? 4 : (mixed && kind == 0 && opt.reserved[2] != 1) ? 2 : kind;
-    // x and r stay in tensor memory when every CTA's rows fit it, the ring
-    // holds the vector passes' copies, and one CTA runs per SM (each CTA
-    // allocates all of the SM's tensor memory)
     // small systems: the matrix stays in the ring, the vectors in registers
     if (!mixed && (launch_kind <= 1 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1)
         launch_kind = launch_kind == 4 ? 8 : launch_kind == 1 ? 9 : 7;
+    // x and r stay in tensor memory when every CTA's rows fit it, the ring
+    // holds the vector passes' copies, and at most one CTA runs per SM (each CTA
+    // allocates all of the SM's tensor memory)
     if ((launch_kind == 2 || launch_kind == 4 || (launch_kind == 0 && !mixed)) && opt.reserved[5] != 1 &&
-        t->G == t->nsm && !(launch_kind == 0 && t->L64.direct)) {
+        t->G <= t->nsm && !(launch_kind == 0 && t->L64.direct)) {
         int rows_max = 0;
         for (size_t g = 0; g + 1 < t->h_cta_rb.size(); ++g)
             rows_max = std::max(rows_max, 16 * (t->h_cta_rb[g + 1] - t->h_cta_rb[g]));

@@ -1169,9 +1169,9 @@ int build_layout(mf_tiles *t, Layout &L, const std::vector<uint8_t> &prec_in, cu
     L.kind = kind;
     L.x32 = x32;
     L.direct = direct;
-    int slabs_max = 0;
-    for (int g = 0; g < G; ++g) slabs_max = std::max(slabs_max, hcnt[g].nslabs);
-    L.resident = !mixed && n_gather == 0 && n_over == 0 && slabs_max <= STAGES && rbps <= RB_PER_SLAB_X64;
+    L.slabs_max = 0;
+    for (int g = 0; g < G; ++g) L.slabs_max = std::max(L.slabs_max, hcnt[g].nslabs);
+    L.resident = !mixed && n_gather == 0 && n_over == 0 && L.slabs_max <= STAGES && rbps <= RB_PER_SLAB_X64;
     L.bytes = off;
     L.alg_bytes = alg;
     for (int p = 0; p < 4; ++p) L.tile_frac[p] = tilenum > 0 ? cnt[p] / tilenum : 0.0;

@@ -246,7 +246,7 @@ struct Layout {
     DevArray<uint8_t> prec_dev;  // per tile precision
     DevArray<float> scale_dev;   // per tile scale (FP16 / FP8)
     std::vector<uint8_t> prec;   // host copy of the precisions
-    int G = 0, nslabs = 0, n_gather = 0, n_oversize = 0;
+    int G = 0, nslabs = 0, n_gather = 0, n_oversize = 0, slabs_max = 0;  // slabs_max: of one CTA
     int slab_max = 0, rb_per_slab = 0;  // stage size / row blocks the planner used
     bool mixed = false;                  // plane precision info present
     int kind = 0;                        // LAYOUT_*
@@ -268,7 +268,7 @@ struct mf_tiles {
     int rowA = 0, colA = 0, tilem = 0, tilen = 0, tilenum = 0, csrsize = 0, csrptrlen = 0;
     int cnt_non_new = 0;
     int device = 0, nsm = 0, l2_bytes = 0;
-    int G = 0;  // persistent CTAs
+    int G = 0;  // persistent CTAs (one an SM; fewer for small FP64 systems)
     mf_options opt;
     bool all_gather = false;  // plan the FP64 layout in gather mode only (batched systems)
     // Tile_create arrays (device); tile_off is tile_nnz == blknnz == csr_offset
