@@ -59,3 +59,25 @@ def test_resident_bicgstab_matches_global_vectors(mf, N):
         x, r = t.solve_bicgstab(b, tol=1e-10, maxiter=2000, opts=mf.options(fixed_iterations=5))
         assert r["iterations"] == 5
         assert np.linalg.norm(x - xg) <= 1e-12 * np.linalg.norm(xg)
+
+
+# 28 row blocks a CTA, 16 CTAs at least, up to 3/4 of the 148 SMs
+@pytest.mark.parametrize("N,ctas", [(4, 16), (84, 16), (85, 17), (222, 111), (224, 148)])
+def test_small_systems_take_few_ctas(mf, O, N, ctas):
+    A = mf.Matrix.poisson2d(N)
+    rp, ci, v = A.csr()
+    b = np.random.default_rng(N).standard_normal(A.n)
+    t = mf.Tiles(A)
+    assert t.info()["nctas"] == ctas
+    o = O.OracleTiles(A.n, A.n, rp, ci, v)
+    assert np.array_equal(t.spmv(b), o.spmv(b))
+    x, r = t.solve_cg(b, tol=1e-10, maxiter=20000)
+    it_o, x_o, _ = o.cg(b, 1e-10, 20000)
+    assert r["status"] == 0 and r["rel_residual_true"] <= 1.5e-10
+    assert abs(r["iterations"] - it_o) <= max(2, 0.02 * it_o)
+
+
+def test_long_rows_and_mixed_handles_keep_every_sm(mf):
+    assert mf.Tiles(mf.Matrix.spd_random(1500, 3)).info()["nctas"] == 148
+    t = mf.Tiles(mf.Matrix.poisson2d(60), mf.options(precision_mode=mf.MODE_MIXED_RULE))
+    assert t.info()["nctas"] == 148
