@@ -52,7 +52,7 @@ struct __align__(16) Smem {
     // thread 0's tallies of a mixed solve (in shared memory: the fences drop
     // spilled registers and local arrays from L1)
     int it_layout[KMAX_LAYOUTS], n_repl, n_switch, fellback;
-    double chunk[PACKET_VALUES * MAX_CHUNKS];  // group_sum: sums of 32 CTAs' packets
+    double chunk[PACKET_VALUES * MAX_CHUNKS];  // group_sum: the polling warps' sums
     uint8_t head[KMAX_LAYOUTS][STAGES][ISSUE_REC];
 };
 
@@ -787,12 +787,40 @@ struct Ctx {
     uint64_t limit_ns;
 };
 
+// Every 64th poll of a wait: true when it ends without what it waits for,
+// because another CTA failed or the time limit passed. t0: 0 before the first.
+__device__ __forceinline__ bool poll_expired(const Ctx &X, Smem &S, uint32_t spin, uint64_t &t0, uint32_t site) {
+    if ((spin & 63u) != 0) return false;
+    if (t0 == 0) t0 = globaltimer();
+    if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
+        S.abort = 1;
+        return true;
+    }
+    if (globaltimer() - t0 > X.limit_ns) {
+        set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, site);
+        S.abort = 1;
+        return true;
+    }
+    return false;
+}
+
 // Sums NV partials over the block and then over the group, in fixed orders:
 // every CTA holds the identical sums. Thread k < NV adds the warps' shares of
 // value k and stores {share of this CTA, phase tag} as one 16-byte packet
-// (slot [phase & 1][rank][k]). Then each warp takes a chunk of CTAs of one
-// value, polls a packet a lane until it carries the tag, and adds the chunk
-// by a shuffle tree; the chunks are added in ascending order.
+// (slot [phase & 1][rank][k]). The G shares of a value are then added as one
+// warp would: lane l takes ranks l, l + 32, l + 64, ... in turn, and a xor
+// tree over the lanes (16, 8, 4, 2, 1) adds the 32 sums. That order is part
+// of the result: a solve that stops on its residual (above all the mixed CG,
+// whose replacements and restarts depend on it) returns another x for another
+// order. To poll the packets in parallel all the same, eight warps share a
+// value: warp s of them takes the ranks = s mod 8, lane l of it the rank
+// s + 8 (l & 3) + 32 (l >> 2). A lane then adds the ranks of its residue mod
+// 32 by shuffles in ascending order, the tree's steps 16 and 8 stay inside the
+// warp, and every thread adds the eight warps' results as steps 4, 2 and 1
+// would. Of four values, each has four warps (ranks = s mod 4) and a lane two
+// packets in flight: eight warps would take two values in turn. us an
+// iteration with a tree for each 32 polled ranks instead, and so: CG 64^3
+// 10.1, 8.7; 50^3 8.0, 7.3; BiCGSTAB 64^3 14.3, 14.5; mixed CG 100^3 19.6, 19.6.
 // Latency-bound: a packet costs one store and one load through L2, where an
 // arrival counter costs a release, the wait on the counter and a second trip
 // for the partials (148 CTAs, 512 threads, one value: 1.4 us against 2.3).
@@ -807,7 +835,7 @@ struct Ctx {
 // stored.
 template <int NV>
 __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (&out)[NV], uint32_t &phase) {
-    static_assert(NV <= PACKET_VALUES, "one packet per value");
+    static_assert(NV <= PACKET_VALUES && NWARPS + 1 == 16, "a packet per value; 16 warps poll");
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -828,79 +856,64 @@ __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (
     // polls that start before the CTA's own store is out only delay the
     // others' stores (1.66 us without this barrier, 1.35 with it)
     __syncthreads();
-    int nch;  // chunks of a value
     if constexpr (NV == 4) {
-        // 20 chunks of 32 would give some warps two in turn: four warps a
-        // value, two packets a lane at once (us an iteration: mixed CG 128^3
-        // 29.8 -> 28.9, BiCGSTAB 64^3 15.0 -> 14.2)
-        nch = 4;
-        const int span = (X.G + 3) >> 2, lo = (w & 3) * span, hi = min(X.G, lo + span);
         double a = 0.0;
-        for (int c = lo + lane; c < hi; c += 64) {
-            const double *p1 = slot + (size_t)c * PACKET_STRIDE + 2 * (w >> 2), *p2 = p1 + 32 * PACKET_STRIDE;
-            bool need1 = true, need2 = c + 32 < hi;
+#pragma unroll 1
+        for (int base = 0; base < X.G; base += 256) {
+            const int c = base + (w & 3) + 4 * (lane & 7) + 32 * (lane >> 3);
+            const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * (w >> 2);
+            bool need1 = c < X.G, need2 = c + 128 < X.G;
             double v1 = 0.0, v2 = 0.0;
             uint64_t t0 = 0;
-            for (uint32_t spin = 1;; ++spin) {
+            for (uint32_t spin = 1; need1 || need2; ++spin) {
                 double u1 = 0.0, u2 = 0.0;
-                const uint64_t g1 = need1 ? ld_packet_relaxed(p1, u1) : 0u, g2 = need2 ? ld_packet_relaxed(p2, u2) : 0u;
+                const uint64_t g1 = need1 ? ld_packet_relaxed(pk, u1) : 0u,
+                               g2 = need2 ? ld_packet_relaxed(pk + 128 * PACKET_STRIDE, u2) : 0u;
                 if (g1 == tag) v1 = u1, need1 = false;
                 if (g2 == tag) v2 = u2, need2 = false;
-                if (!need1 && !need2) break;
-                if ((spin & 63u) == 0) {
-                    if (t0 == 0) t0 = globaltimer();
-                    if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
-                        S.abort = 1;
-                        break;
-                    }
-                    if (globaltimer() - t0 > X.limit_ns) {
-                        set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, 10);
-                        S.abort = 1;
-                        break;
-                    }
-                }
+                if ((need1 || need2) && poll_expired(X, S, spin, t0, 10)) break;
             }
-            a += v1 + v2;
-        }
-        __syncwarp();
+            __syncwarp();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            for (int j = 0; j < 4; ++j)
+                if (base + 32 * j < X.G) a += __shfl_sync(0xffffffffu, v1, 8 * j + (lane & 7));
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (base + 128 + 32 * j < X.G) a += __shfl_sync(0xffffffffu, v2, 8 * j + (lane & 7));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (lane == 0) S.chunk[w] = a;
     } else {
-        nch = (X.G + 31) >> 5;
-        for (int ch = w; ch < NV * nch; ch += NWARPS + 1) {
-            const int k = ch / nch, c = (ch - k * nch) * 32 + lane;
-            __syncwarp();
+        for (int ch = w; ch < 8 * NV; ch += NWARPS + 1) {
             double a = 0.0;
-            if (c < X.G) {
-                const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * k;
-                uint64_t t0 = 0;
-                for (uint32_t spin = 1; ld_packet_relaxed(pk, a) != tag; ++spin) {
-                    // a pause between polls: the polls of the CTAs that wait
-                    // share L2 with the stores they wait for. us an iteration
-                    // with and without: 5-point CG 256^2 5.6..6.0, 5.8..7.3;
-                    // Jacobi PCG 75^3 14.3..14.9, 14.5..16.4; FP64 CG 128^3
-                    // 38.0, 38.4; not with four values (mixed CG 29.9, 29.7)
-                    const long long t1 = clock64();
-                    while (clock64() - t1 < 150) {
-                    }
-                    if ((spin & 63u) == 0) {
-                        if (t0 == 0) t0 = globaltimer();
-                        if (ld_relaxed(X.sync + SYNC_ERROR) != 0u) {
-                            S.abort = 1;
-                            break;
+#pragma unroll 1
+            for (int base = 0; base < X.G; base += 256) {
+                const int c = base + (w & 7) + 8 * (lane & 3) + 32 * (lane >> 2);
+                const double *pk = slot + (size_t)c * PACKET_STRIDE + 2 * (ch >> 3);
+                double u = 0.0;
+                if (c < X.G) {
+                    uint64_t t0 = 0;
+                    for (uint32_t spin = 1; ld_packet_relaxed(pk, u) != tag; ++spin) {
+                        // a pause between polls: the polls of the CTAs that wait
+                        // share L2 with the stores they wait for. us an iteration
+                        // with and without: 5-point CG 256^2 5.6..6.0, 5.8..7.3;
+                        // Jacobi PCG 75^3 14.3..14.9, 14.5..16.4; FP64 CG 128^3
+                        // 38.0, 38.4; not with four values (mixed CG 29.9, 29.7)
+                        const long long t1 = clock64();
+                        while (clock64() - t1 < 150) {
                         }
-                        if (globaltimer() - t0 > X.limit_ns) {
-                            set_error_w(X.sync, (uint32_t)MF_ERR_TIMEOUT, 10);
-                            S.abort = 1;
-                            break;
-                        }
+                        if (poll_expired(X, S, spin, t0, 10)) break;
                     }
                 }
+                __syncwarp();
+                // rolled: unrolled, CG 64^3 takes 9.0 us an iteration, so 8.7
+#pragma unroll 1
+                for (int j = 0; j < 8 && base + 32 * j < X.G; ++j)
+                    a += __shfl_sync(0xffffffffu, u, 4 * j + (lane & 3));
             }
-            __syncwarp();
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            a += __shfl_xor_sync(0xffffffffu, a, 2);
+            a += __shfl_xor_sync(0xffffffffu, a, 1);
             if (lane == 0) S.chunk[ch] = a;
         }
     }
@@ -908,9 +921,13 @@ __device__ bool group_sum(const Ctx &X, Smem &S, const double (&v)[NV], double (
     if (S.abort) return false;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        double a = S.chunk[k * nch];
-        for (int ch = 1; ch < nch; ++ch) a += S.chunk[k * nch + ch];
-        out[k] = a;
+        if constexpr (NV == 4) {
+            const double *c = S.chunk + 4 * k;
+            out[k] = (c[0] + c[2]) + (c[1] + c[3]);
+        } else {
+            const double *c = S.chunk + 8 * k;
+            out[k] = ((c[0] + c[4]) + (c[2] + c[6])) + ((c[1] + c[5]) + (c[3] + c[7]));
+        }
     }
     ++phase;
     return true;
