@@ -52,7 +52,7 @@ struct __align__(16) Smem {
     // thread 0's tallies of a mixed solve (in shared memory: the fences drop
     // spilled registers and local arrays from L1)
     int it_layout[KMAX_LAYOUTS], n_repl, n_switch, fellback;
-    double chunk[PACKET_VALUES * MAX_CHUNKS];  // group_sum: the polling warps' sums
+    double chunk[SUM_CHUNKS];  // group_sum: the polling warps' sums
     uint8_t head[KMAX_LAYOUTS][STAGES][ISSUE_REC];
 };
 
@@ -3545,7 +3545,6 @@ int kernel_config(mf_tiles *t, int *G_out) {
     int per_sm = t->opt.ctas_per_sm > 0 ? t->opt.ctas_per_sm : 1;
     if (per_sm > occ_min) per_sm = occ_min;
     *G_out = t->nsm * per_sm;
-    if (*G_out > 32 * MAX_CHUNKS) *G_out = 32 * MAX_CHUNKS;  // group_sum's chunk sums
     return MF_OK;
 }
 

@@ -20,7 +20,7 @@ enum { SYNC_ERROR = 32, SYNC_SITE = 33, SYNC_FLAGS = 64 };
 // slots x G CTAs x PACKET_STRIDE doubles (a 128-byte line), of which
 // PACKET_VALUES {value, phase tag} pairs are used.
 constexpr int PACKET_VALUES = 4, PACKET_STRIDE = 16;
-constexpr int MAX_CHUNKS = 32;  // of 32 CTAs: grids of up to 1024 CTAs
+constexpr int SUM_CHUNKS = 24;  // warps' sums of one group_sum: 4 values x 4 warps, up to 3 values x 8
 __host__ __device__ inline size_t partial_words(int G) { return 2 * PACKET_STRIDE * (size_t)G; }
 inline size_t sync_words(int G) { return (size_t)SYNC_FLAGS + (size_t)G * FLAG_STRIDE + 32; }
 
