@@ -508,11 +508,14 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
             const int k = i % STAGES;
             uint8_t *st = stage_ptr(dyn, k, stride);
             if ((pp.filled >> k) & 1u) {
-                if (!wait_bar(&S.empty[k], (pp.eph >> k) & 1u, C.limit_ns)) {
+                const bool ok = wait_bar(&S.empty[k], (pp.eph >> k) & 1u, C.limit_ns);
+                if (!ok) {
                     set_error_w(C.sync, (uint32_t)MF_ERR_TIMEOUT, 110 + L.site);
                     S.abort = 1;
-                    break;
                 }
+                // each lane has its own clock: the warp leaves together, or a
+                // lane that ran out would miss the warp barriers below
+                if (!__all_sync(0xffffffffu, ok)) break;
                 pp.eph ^= 1u << k;
             }
             pp.filled |= 1u << k;
