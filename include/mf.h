@@ -82,6 +82,8 @@ typedef struct {
     int reserved[7];         /* reserved[0] == 0x5741: test hook, the CG kernel
                                 first waits on a flag nothing sets, so the
                                 bounded wait must end it with MF_ERR_TIMEOUT;
+                                0x5742: the same in a later iteration of the
+                                kernels of small systems;
                                 reserved[1] = N > 0: trace the first N CG
                                 iterations (see mf_trace); reserved[2] = 1:
                                 mixed layouts use the classic two-reduction

@@ -507,7 +507,7 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     P.fixed_iterations = opt.fixed_iterations;
     P.replace_every = opt.replace_every;
     P.res = v.res;
-    P.inject_wait = opt.reserved[0] == 0x5741 ? 1 : 0;
+    P.inject_wait = opt.reserved[0] == 0x5741 ? 1 : opt.reserved[0] == 0x5742 ? 2 : 0;
     P.prefetch = opt.reserved[3] == 1 ? 1 : 0;
     if (opt.reserved[1] > 0) {
         const int ti = opt.reserved[1] > 4096 ? 4096 : opt.reserved[1];

@@ -1154,7 +1154,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg(KParams P) {
     double *x = P.x, *r = P.r, *d = P.d, *q = P.q;
     float *d32 = MIXED ? reinterpret_cast<float *>(P.t) : nullptr;  // FP32 d for FP32-x layouts
     const double *b = P.b;
-    if (P.inject_wait) {
+    if (P.inject_wait == 1) {
         // test hook: a dependency epoch no CTA ever publishes; the bounded
         // wait must end the solve with MF_ERR_TIMEOUT
         if (!wait_deps(P, S, 0, 0xffffffffu)) return;
@@ -2274,7 +2274,7 @@ __device__ __forceinline__ void cg_tm_body(const KParams &P, Smem &S, uint8_t *d
     double *x = P.x, *r = P.r, *d = P.d, *q = P.q;
     const double *b = P.b;
     const double *sv = reinterpret_cast<const double *>(dyn);
-    if (P.inject_wait) {
+    if (P.inject_wait == 1) {
         // test hook (as in k_cg): an epoch no CTA publishes; the bounded wait
         // must end the solve with MF_ERR_TIMEOUT
         if (!wait_deps(P, S, 0, 0xffffffffu)) return;
@@ -2660,6 +2660,7 @@ __device__ __forceinline__ void res_spmv(const KParams &P, Smem &S, uint8_t *dyn
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (w == PRODUCER_WARP) {
         const Ctx X = ctx_of(P);
+        if (P.inject_wait == 2 && ep > 2u) ep = 0xffffffffu;  // test hook
         const bool ok = ep == 0u || poll_deps(X, S, P.lay[0].cta_dep[2 * blockIdx.x],
                                               P.lay[0].cta_dep[2 * blockIdx.x + 1], ep);
         if (__all_sync(0xffffffffu, ok)) {
@@ -2681,6 +2682,11 @@ __device__ __forceinline__ void res_spmv(const KParams &P, Smem &S, uint8_t *dyn
                              (uint32_t)run.nseg * 128u, &S.full[i], pv);
                 }
             }
+        } else if (lane == 0) {
+            // no copy will land: the consumers go on over the old windows to
+            // the next grid sum, which ends on S.abort, instead of waiting
+            // out a time limit of their own
+            for (int i = 0; i < ns; ++i) mbar_arrive(&S.full[i]);
         }
     } else {
         const int j = 2 * w + (lane >> 4), r = lane & 15;
@@ -2716,7 +2722,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_cg_res(KParams P) {
     kernel_setup(P, S, 1);
     const int g = blockIdx.x, tid = threadIdx.x;
     uint32_t phase = 0, par = 0;
-    if (P.inject_wait) {
+    if (P.inject_wait == 1) {
         // test hook (as in k_cg): an epoch no CTA publishes
         if (!wait_deps(P, S, 0, 0xffffffffu)) return;
     }

@@ -61,7 +61,8 @@ struct KParams {
     const double *b;
     double tol;
     int maxiter, fixed_iterations, replace_every;
-    int inject_wait;  // test hook: wait once on a flag that nothing sets
+    int inject_wait;  // test hook: wait on a flag that nothing sets, 1 before the first SpMV, 2 in a
+                      // later one of the resident kernels (by their producer warp)
     int true_check;   // confirm convergence with the FP64 true residual
     int trace_iters;  // CTA 0 records %globaltimer at each phase boundary
     int prefetch;     // L2 bulk prefetch of slabs ahead of the ring
