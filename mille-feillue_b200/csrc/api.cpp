@@ -729,8 +729,11 @@ static int solve_dev(mf_tiles *t, int kind, const double *b_dev, double *x_dev, 
 // Re-plans the handle's layouts (FP64 and, when present, the mixed levels)
 // with the candidate slab geometry and returns the time of the SpMV the
 // solvers run (the mixed level 0 when present, else FP64), averaged over
-// reps launches.
-static int tune_candidate(mf_tiles *t, int slab_bytes, int rbps, int reps, double *ms) {
+// reps launches. set: the precisions of mf_tiles_set_precisions on an FP64
+// handle, or empty; their layout shares the FP64 layout's stages and is
+// planned again with it.
+static int tune_candidate(mf_tiles *t, int slab_bytes, int rbps, int reps, const std::vector<uint8_t> &set,
+                          double *ms) {
     t->opt.slab_bytes = slab_bytes;
     t->opt.rb_per_slab = rbps;
     int G = 0, rc;
@@ -739,6 +742,10 @@ static int tune_candidate(mf_tiles *t, int slab_bytes, int rbps, int reps, doubl
     if ((rc = build_layout(t, t->L64, prec, 0)) != MF_OK) return rc;
     const bool mixed = t->opt.precision_mode != MF_MODE_FP64;
     if (mixed && (rc = build_mixed_levels(t, 0)) != MF_OK) return rc;
+    if (!set.empty()) {
+        if ((rc = build_layout(t, t->Lmix[0], set, 0)) != MF_OK) return rc;
+        t->Lbicg.built = false;
+    }
     const int level = (mixed && t->mixed_ready) ? 0 : -1;
     if ((rc = ensure_workspace(t)) != MF_OK) return rc;
     WsView v = ws_view(t);
@@ -772,6 +779,8 @@ int mf_tiles_autotune(mf_tiles *t, int reps, mf_tune_result *out) {
     if (reps <= 0) reps = 20;
     MF_CUDA_TRY(cudaSetDevice(t->opt.device));
     std::memset(out, 0, sizeof *out);
+    std::vector<uint8_t> set;
+    if (t->opt.precision_mode == MF_MODE_FP64 && t->mixed_ready) set = t->Lmix[0].prec;
     static const int kSlab[] = {24576, 32768, 40960};
     static const int kRb[] = {16, 30, 60, 120};
     double best = 1e30;
@@ -779,7 +788,7 @@ int mf_tiles_autotune(mf_tiles *t, int reps, mf_tune_result *out) {
     for (int sb : kSlab)
         for (int rb : kRb) {
             double ms = 0;
-            const int rc = tune_candidate(t, sb, rb, reps, &ms);
+            const int rc = tune_candidate(t, sb, rb, reps, set, &ms);
             if (rc == MF_ERR_ARG) continue;  // does not fit shared memory
             if (rc) return rc;
             const int k = out->candidates++;
@@ -797,7 +806,7 @@ int mf_tiles_autotune(mf_tiles *t, int reps, mf_tune_result *out) {
         }
     if (out->candidates == 0) return MF_ERR_RESIDENCY;
     double ms = 0;
-    int rc = tune_candidate(t, bsb, brb, reps, &ms);  // leave the handle on the choice
+    int rc = tune_candidate(t, bsb, brb, reps, set, &ms);  // leave the handle on the choice
     if (rc) return rc;
     out->slab_bytes = bsb;
     out->rb_per_slab = brb;
