@@ -83,6 +83,33 @@ int ensure_host_tiles(const mf_tiles *t) {
     return MF_OK;
 }
 
+// Plans the FP64 layout of a handle that may use up to g_all CTAs, and with it
+// the handle's CTA count.
+// A small FP64 system takes about one full slab a CTA instead of every
+// SM: its solves are bound by the grid sums, which cost more the more CTAs
+// poll (us an iteration with 148 CTAs and so: 5-point CG 37^2 5.5 -> 5.0,
+// 90^2 5.9 -> 5.0; Jacobi PCG 13^3 8.5 -> 5.3; BiCGSTAB 16^3 10.7 -> 7.6;
+// below 16 CTAs little changes, and the SpMV alone slows down). 28 row
+// blocks a CTA on average leave every range within the slab's 30. Not for
+// scattered matrices (about one entry a tile) or rows so long that 28 row
+// blocks need a second slab: those want every SM, and where the estimate
+// errs the layout is planned again.
+static int plan_fp64(mf_tiles *t, int g_all, cudaStream_t s) {
+    const std::vector<uint8_t> prec(t->tilenum, MF_PREC_FP64);
+    const int g_few = std::max(16, (t->tilem + 27) / 28);
+    auto plan = [&](int G) -> int {
+        if (t->G != G) t->h_cta_rb.clear();
+        t->G = G;
+        return build_layout(t, t->L64, prec, s);
+    };
+    if (t->opt.precision_mode == MF_MODE_FP64 && 4 * g_few <= 3 * g_all && t->csrsize >= 2ll * t->tilenum &&
+        12.0 * 28.0 * t->csrsize <= (double)SLAB_MAX_DEFAULT * t->tilem) {
+        const int rc = plan(g_few);
+        if (rc || (t->L64.resident && t->L64.slabs_max <= 1)) return rc;
+    }
+    return plan(g_all);
+}
+
 // Encodes a device CSR; G > 0 forces the number of CTA ranges of the layout
 // (the CTAs of a group, for the batched solver), all_gather a layout in gather
 // mode only.
@@ -102,26 +129,9 @@ int encode_dev_impl(int n, int ncols, int nnz, const int *rp, const int *ci, con
     if (G_force > 0) t->G = G_force;
     cudaStream_t s = 0;
     if ((rc = encode_device(t, n, ncols, nnz, rp, ci, val, s)) != MF_OK) { delete t; return rc; }
-    std::vector<uint8_t> prec(t->tilenum, MF_PREC_FP64);
-    // A small FP64 system takes about one full slab a CTA instead of every
-    // SM: its solves are bound by the grid sums, which cost more the more CTAs
-    // poll (us an iteration with 148 CTAs and so: 5-point CG 37^2 5.5 -> 5.0,
-    // 90^2 5.9 -> 5.0; Jacobi PCG 13^3 8.5 -> 5.3; BiCGSTAB 16^3 10.7 -> 7.6;
-    // below 16 CTAs little changes, and the SpMV alone slows down). 28 row
-    // blocks a CTA on average leave every range within the slab's 30. Not for
-    // scattered matrices (about one entry a tile) or rows so long that 28 row
-    // blocks need a second slab: those want every SM, and where the estimate
-    // errs the layout is planned again.
-    const int g_all = t->G, g_few = std::max(16, (t->tilem + 27) / 28);
-    if (G_force == 0 && t->opt.precision_mode == MF_MODE_FP64 && 4 * g_few <= 3 * g_all &&
-        t->csrsize >= 2ll * t->tilenum && 12.0 * 28.0 * t->csrsize <= (double)SLAB_MAX_DEFAULT * t->tilem)
-        t->G = g_few;
-    if ((rc = build_layout(t, t->L64, prec, s)) != MF_OK) { delete t; return rc; }
-    if (t->G < g_all && !(t->L64.resident && t->L64.slabs_max <= 1)) {
-        t->G = g_all;
-        t->h_cta_rb.clear();
-        if ((rc = build_layout(t, t->L64, prec, s)) != MF_OK) { delete t; return rc; }
-    }
+    if (G_force > 0) rc = build_layout(t, t->L64, std::vector<uint8_t>(t->tilenum, MF_PREC_FP64), s);
+    else rc = plan_fp64(t, t->G, s);
+    if (rc != MF_OK) { delete t; return rc; }
     if (t->opt.precision_mode != MF_MODE_FP64) {
         if ((rc = build_mixed_levels(t, s)) != MF_OK) { delete t; return rc; }
     }
@@ -738,8 +748,7 @@ static int tune_candidate(mf_tiles *t, int slab_bytes, int rbps, int reps, const
     t->opt.rb_per_slab = rbps;
     int G = 0, rc;
     if ((rc = kernel_config(t, &G)) != MF_OK) return rc;
-    std::vector<uint8_t> prec(t->tilenum, MF_PREC_FP64);
-    if ((rc = build_layout(t, t->L64, prec, 0)) != MF_OK) return rc;
+    if ((rc = plan_fp64(t, G, 0)) != MF_OK) return rc;
     const bool mixed = t->opt.precision_mode != MF_MODE_FP64;
     if (mixed && (rc = build_mixed_levels(t, 0)) != MF_OK) return rc;
     if (!set.empty()) {

@@ -1171,7 +1171,10 @@ int build_layout(mf_tiles *t, Layout &L, const std::vector<uint8_t> &prec_in, cu
     L.direct = direct;
     L.slabs_max = 0;
     for (int g = 0; g < G; ++g) L.slabs_max = std::max(L.slabs_max, hcnt[g].nslabs);
-    L.resident = !mixed && n_gather == 0 && n_over == 0 && L.slabs_max <= STAGES && rbps <= RB_PER_SLAB_X64;
+    int rb_max = 0;  // row blocks of one CTA
+    for (int g = 0; g < G; ++g) rb_max = std::max(rb_max, cta_rb[g + 1] - cta_rb[g]);
+    L.resident = !mixed && n_gather == 0 && n_over == 0 && L.slabs_max <= STAGES &&
+                 std::min(rbps, rb_max) <= RB_PER_SLAB_X64;  // at most 30 row blocks in any slab
     L.bytes = off;
     L.alg_bytes = alg;
     for (int p = 0; p < 4; ++p) L.tile_frac[p] = tilenum > 0 ? cnt[p] / tilenum : 0.0;
