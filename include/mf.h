@@ -98,7 +98,9 @@ typedef struct {
                                 systems' sizes); reserved[5] = 1:
                                 the solver kernels keep their vectors in
                                 global memory instead of tensor memory or
-                                registers;
+                                registers; 2: CG and Jacobi PCG run the
+                                tensor-memory kernels of large systems on
+                                small and scattered ones too (for tests);
                                 reserved[6] = N > 0: reference iteration
                                 count for the learned selector's fallback   */
 } mf_options;

@@ -589,13 +589,14 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     }
     int launch_kind = kind == 2 ? 4 : (mixed && kind == 0 && opt.reserved[2] != 1) ? 2 : kind;
     // small systems: the matrix stays in the ring, the vectors in registers
-    if (!mixed && (launch_kind <= 1 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1)
+    if (!mixed && (launch_kind <= 1 || launch_kind == 4) && t->L64.resident && opt.reserved[5] != 1 &&
+        opt.reserved[5] != 2)
         launch_kind = launch_kind == 4 ? 8 : launch_kind == 1 ? 9 : 7;
     // x and r stay in tensor memory when every CTA's rows fit it, the ring
     // holds the vector passes' copies, and at most one CTA runs per SM (each CTA
     // allocates all of the SM's tensor memory)
     if ((launch_kind == 2 || launch_kind == 4 || (launch_kind == 0 && !mixed)) && opt.reserved[5] != 1 &&
-        t->G <= t->nsm && !(launch_kind == 0 && t->L64.direct)) {
+        t->G <= t->nsm && !(launch_kind == 0 && t->L64.direct && opt.reserved[5] != 2)) {
         int rows_max = 0;
         for (size_t g = 0; g + 1 < t->h_cta_rb.size(); ++g)
             rows_max = std::max(rows_max, 16 * (t->h_cta_rb[g + 1] - t->h_cta_rb[g]));
