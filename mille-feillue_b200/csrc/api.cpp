@@ -464,19 +464,6 @@ static int true_residual_ws(mf_tiles *t, const double *b, const double *x, doubl
     return MF_OK;
 }
 
-// 1/256ths of a layout's slabs a solve keeps in L2 from one SpMV to the next
-// (LayoutArgs::keep). A layout that with the vectors (about 32 bytes a row)
-// outgrows L2 would, copied with evict_first alone, be read from memory
-// whole every iteration; a quarter of L2 goes to its first slabs. 128^3
-// (126 MB of L2), us an iteration with 0 / 38 / 75 / 150 MB kept: FP64 CG
-// 39.9 / 38.3 / 39.8 / 40.9; mixed CG 30.4 with 0, 29.7 with 14, 30.2 with
-// its whole 55 MB. A layout that fits (75^3: 30 MB) gains nothing.
-static int l2_keep(const mf_tiles *t, const Layout &L) {
-    const double l2 = (double)t->l2_bytes, bytes = (double)L.bytes;
-    if (l2 <= 0.0 || bytes <= 0.0 || bytes + 32.0 * t->rowA <= 0.75 * l2) return 0;
-    return (int)std::min(256.0, 256.0 * 0.25 * l2 / bytes);
-}
-
 // kind 0 = CG, 1 = BiCGSTAB, 2 = Jacobi-preconditioned CG (FP64 layout).
 // b_dev / x_dev: n entries (device). x in: x0.
 static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_dev, double tol, int maxiter,
@@ -498,7 +485,6 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
     MF_CUDA_TRY(cudaMemsetAsync(t->sync.p, 0, sizeof(uint32_t) * t->sync.n));
     KParams P;
     base_params(t, P);
-    P.lay[0].keep = l2_keep(t, t->L64);
     if (opt.timeout_s > 0) P.limit_ns = (uint64_t)(opt.timeout_s * 1e9);
     P.sync = t->sync.p;
     P.partial = v.partial;
@@ -549,7 +535,6 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
             a.cta_dep = L.cta_dep.p;
             a.kind = L.kind;
             a.x32 = L.x32 ? 1 : 0;
-            a.keep = l2_keep(t, L);
             P.level_rel[nl] = rel;
             ++nl;
         };
@@ -618,6 +603,8 @@ static int solve_dev_once(mf_tiles *t, int kind, const double *b_dev, double *x_
         int rj = launch_to_f32((int)n16, v.s, v.p32, n16, 0);
         if (rj) return rj;
     }
+    for (int l = 0; l < P.nlay; ++l)
+        P.lay[l].keep = l2_keep(launch_kind, t->l2_bytes, (double)(l == 0 ? &t->L64 : lv[l - 1])->bytes, n);
     rc = launch_solver(t, launch_kind, P, 0);
     cudaEventRecord(e1, 0);
     // everything after the solve is queued behind it, and one copy waits for

@@ -121,6 +121,23 @@ int launch_to_f32(int n, const double *src, float *dst, size_t npad, cudaStream_
 // BiCGSTAB with the matrix in the ring and the vectors in registers
 // (L64.resident).
 constexpr int TMEM_ROWS_MAX = 128 * 128;
+// 1/256ths of a layout's slabs that a solve by kernel `kind` keeps in L2 from
+// one SpMV to the next (LayoutArgs::keep). A layout that with the vectors
+// outgrows L2 would, copied with evict_first alone, be read from memory whole
+// every iteration; a quarter of L2 goes to its first slabs. Only beside the
+// kernels with x and r in tensor memory, whose other vectors are about 32
+// bytes a row: 128^3 (126 MB of L2), us an iteration with 0 / 38 / 75 / 150 MB
+// kept: FP64 CG 39.9 / 38.3 / 39.8 / 40.9; mixed CG 30.4 with 0, 29.7 with 14,
+// 30.2 with its whole 55 MB. A layout that fits (75^3: 30 MB) gains nothing.
+// The other kernels' vectors are in L2 themselves (56 to 136 bytes a row and
+// iteration), and slabs kept there drive them out: BiCGSTAB 110^3 62.4 with 0,
+// 71.7 with a quarter; 128^3: Jacobi PCG 48.7, 57.0, classic mixed CG 50.1, 54.9.
+inline int l2_keep(int kind, double l2, double bytes, double rows) {
+    if (kind != 3 && kind != 5 && kind != 6) return 0;
+    if (l2 <= 0.0 || bytes <= 0.0 || bytes + 32.0 * rows <= 0.75 * l2) return 0;
+    const double share = 256.0 * 0.25 * l2 / bytes;
+    return share < 256.0 ? (int)share : 256;
+}
 // The TMEM kernel's vector pass copies 12 bytes per own row into the ring.
 inline bool tm_vectors_fit(int rows_max, int slab_max) {
     return 12ll * rows_max <= (long long)STAGES * stage_stride_of(slab_max);
