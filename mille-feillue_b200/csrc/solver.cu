@@ -3542,7 +3542,12 @@ int kernel_config(mf_tiles *t, int *G_out) {
                            (const void *)k_cg_res<true>, (const void *)k_bicgstab_res};
     int occ_min = 1 << 30;
     for (const void *k : kerns) {
-        MF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+        // the kernel's limit, not this handle's need: the launches of handles
+        // with larger slabs go through the same attribute
+        cudaFuncAttributes fa;
+        MF_CUDA_TRY(cudaFuncGetAttributes(&fa, k));
+        MF_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         optin - (int)fa.sharedSizeBytes));
         int occ = 0;
         MF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, NTHREADS, dyn));
         occ_min = occ < occ_min ? occ : occ_min;
