@@ -83,6 +83,11 @@ int ensure_host_tiles(const mf_tiles *t) {
     return MF_OK;
 }
 
+static int plan_fp64_on(mf_tiles *t, int G, cudaStream_t s) {
+    if (t->G != G) t->h_cta_rb.clear();
+    t->G = G;
+    return build_layout(t, t->L64, std::vector<uint8_t>(t->tilenum, MF_PREC_FP64), s);
+}
 // Plans the FP64 layout of a handle that may use up to g_all CTAs, and with it
 // the handle's CTA count.
 // A small FP64 system takes about one full slab a CTA instead of every
@@ -93,21 +98,17 @@ int ensure_host_tiles(const mf_tiles *t) {
 // blocks a CTA on average leave every range within the slab's 30. Not for
 // scattered matrices (about one entry a tile) or rows so long that 28 row
 // blocks need a second slab: those want every SM, and where the estimate
-// errs the layout is planned again.
+// errs the layout is planned again. Not with low-precision layouts either
+// (mf_tiles_set_precisions): their solves decide on the grid sums, whose
+// rounding follows the CTA count.
 static int plan_fp64(mf_tiles *t, int g_all, cudaStream_t s) {
-    const std::vector<uint8_t> prec(t->tilenum, MF_PREC_FP64);
     const int g_few = std::max(16, (t->tilem + 27) / 28);
-    auto plan = [&](int G) -> int {
-        if (t->G != G) t->h_cta_rb.clear();
-        t->G = G;
-        return build_layout(t, t->L64, prec, s);
-    };
-    if (t->opt.precision_mode == MF_MODE_FP64 && 4 * g_few <= 3 * g_all && t->csrsize >= 2ll * t->tilenum &&
-        12.0 * 28.0 * t->csrsize <= (double)SLAB_MAX_DEFAULT * t->tilem) {
-        const int rc = plan(g_few);
+    if (t->opt.precision_mode == MF_MODE_FP64 && !t->mixed_ready && 4 * g_few <= 3 * g_all &&
+        t->csrsize >= 2ll * t->tilenum && 12.0 * 28.0 * t->csrsize <= (double)SLAB_MAX_DEFAULT * t->tilem) {
+        const int rc = plan_fp64_on(t, g_few, s);
         if (rc || (t->L64.resident && t->L64.slabs_max <= 1)) return rc;
     }
-    return plan(g_all);
+    return plan_fp64_on(t, g_all, s);
 }
 
 // Encodes a device CSR; G > 0 forces the number of CTA ranges of the layout
@@ -303,8 +304,11 @@ int mf_tiles_set_precisions(mf_tiles *t, const unsigned char *prec) {
     std::vector<uint8_t> p(prec, prec + t->tilenum);
     for (auto &v : p)
         if (v > MF_PREC_FP8) return MF_ERR_ARG;
-    int rc = build_layout(t, t->Lmix[0], p, 0);
-    if (rc) return rc;
+    // the layouts of a handle share its CTA ranges: mixed solves take every SM
+    int g_all = 0, rc;
+    if ((rc = kernel_config(t, &g_all)) != MF_OK) return rc;
+    if (t->G < g_all && (rc = plan_fp64_on(t, g_all, 0)) != MF_OK) return rc;
+    if ((rc = build_layout(t, t->Lmix[0], p, 0)) != MF_OK) return rc;
     for (int l = 1; l < MF_NLEVELS; ++l) t->Lmix[l].built = false;
     t->Lbicg.built = false;
     t->nlevels = 1;
