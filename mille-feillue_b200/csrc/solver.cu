@@ -476,6 +476,15 @@ __device__ double global_row(const GTiles &P, int rb, int r, const double *__res
     return acc;
 }
 
+// The same as a call, for the kernels with GB > 1 (the standalone SpMV and the
+// batch): inlined into their pipeline the loop is slower. SpMV of 3000 rows,
+// two of about 2300 entries: 225 us inlined, 201 as a call; batch of 12 random
+// systems of 20000 rows, some of over 400 entries, in groups of 4: 2441 ms,
+// 2068. The other solvers keep it inlined: a call makes them spill.
+__device__ __noinline__ double global_row_call(const GTiles P, int rb, int r, const double *xg) {
+    return global_row(P, rb, r, xg);
+}
+
 // Tiled SpMV of this CTA's row range with layout `lay` and input vector xv.
 // Warp PRODUCER_WARP streams the CTA's slabs into the STAGES-deep ring: it
 // waits until the consumers released a stage, then issues the slab and the x
@@ -585,7 +594,9 @@ __device__ bool cta_spmv_src(const SpmvSrc &L, const PipeCfg &C, const void *xv,
                     const int row = h.rb0 * 16 + r;
                     using PV = decltype(epi.pre(0));
                     const PV pv = row < L.gt.rowA ? epi.pre(row) : PV(0);
-                    const double acc = global_row(L.gt, h.rb0, r, static_cast<const double *>(xv));
+                    double acc;
+                    if constexpr (GB > 1) acc = global_row_call(L.gt, h.rb0, r, static_cast<const double *>(xv));
+                    else acc = global_row(L.gt, h.rb0, r, static_cast<const double *>(xv));
                     if (row < L.gt.rowA) epi(row, acc, pv);
                 }
             } else {
