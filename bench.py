@@ -373,7 +373,7 @@ def gpu_arm(args, world, rank, local, dist):
     # (dram__bytes_read + write; profiles/k_cg_tm_k_cgcg_tm_varpoisson128.md),
     # scaled by the iterations of the timed solve (plus the initial and the
     # replacement FP64 SpMVs at their algorithmic bytes)
-    dram_per_iter = {"mixed": 15.0e6, "fp64": 122.6e6}[headline]
+    dram_per_iter = {"mixed": 13.9e6, "fp64": 129.0e6}[headline]
     traffic = res["iterations"] * dram_per_iter + (1 + res["replacements"]) * spmv_bytes
     kname = ("k_cgcg_tm (mixed single-reduction CG, x and r in tensor memory)" if headline == "mixed"
              else "k_cg_tm (FP64 CG, x and r in tensor memory)")

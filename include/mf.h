@@ -220,7 +220,8 @@ int mf_tiles_export(const mf_tiles *t, mf_tile_arrays *host);
 /* Per-tile precision codes (MF_PREC_*) and scales of the current layout.    */
 int mf_tiles_precisions(const mf_tiles *t, unsigned char *prec_host,
                         float *scale_host);
-/* Re-encode the solver layout with explicit per-tile precisions.            */
+/* Re-encode the solver layout with explicit per-tile precisions. A small FP64
+ * handle moves to every SM (nctas), as handles encoded for mixed solves are.  */
 int mf_tiles_set_precisions(mf_tiles *t, const unsigned char *prec_host);
 
 /* Two-pointer warp work split of the reference driver (compatibility

@@ -70,9 +70,14 @@ constexpr int kBatchGroupMin = 4;  // smallest group the rule below considers
 // kNnzUs * nnz / gs (scattered systems, whose gathers bound them; equal
 // iteration counts). Small groups keep every CTA busy when there are many
 // systems (512 of 1e3..2e5 rows: 4 CTAs); with few, the largest system alone
-// would hold the launch (48 such systems: 74.2 ms in groups of 4, 21.2 in 16,
-// 26.1 in 37, 22.2 in the chosen 13; 3 systems: 32.5 ms in 4, 4.3 in 37, 2.7
-// in the chosen 148).
+// would hold the launch. The two constants were fitted when scattered systems
+// still ran through the copy ring. Measured on the present kernels, to 1e-10:
+// 48 scattered systems of 1e3..2e5 rows 40.7 ms in groups of 4, 12.1 in the
+// chosen 16, 15.6 in 37, 37.8 in 148; 3 of 1e5 rows 18.1 in 4, 2.1 in the
+// chosen 49; 40 5-point grids of 30^2..320^2 76.8 in 4, 35.4 in the chosen
+// 10, 25.4 in 16; 300 of 40^2..200^2 47.1 in the chosen 4, 66.1 in 8. Of 19
+// such sets, grids and scattered, the choice was slower than groups of 4 in
+// none by more than 7 % (12 grids of 20^2: 0.51 ms against 0.48).
 constexpr double kIterUs = 10.0, kNnzUs = 1.1e-3;
 int choose_group(int nsm, std::vector<long long> nnz) {
     std::sort(nnz.begin(), nnz.end(), std::greater<long long>());

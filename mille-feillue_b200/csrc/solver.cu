@@ -15,8 +15,8 @@
 // every CTA polls the G packets until all carry the tag and sums them in the
 // same fixed order, so all CTAs hold the identical value (no grid.sync, no
 // kernel boundary). Vector halos
-// between iterations use per-CTA epoch flags (st.release / ld.acquire) that
-// only the CTAs whose rows a CTA reads are waited on. Every wait is bounded
+// between iterations use per-CTA epoch flags (fence.acq_rel, relaxed store /
+// ld.acquire) that only the CTAs whose rows a CTA reads are waited on. Every wait is bounded
 // by %globaltimer; on expiry the kernel records MF_ERR_TIMEOUT and returns.
 //
 // The recurrences follow Mille-feuille_CG_NVIDIA.cu:722-804 (CG) and
